@@ -472,6 +472,15 @@ int wf_stage_wait_selftest(wf_solver* h, int short_stage, double timeout_ms, int
  * package).  Drops the handle's captured step graphs; rebuild batches that
  * contain the handle afterwards. */
 int wf_set_blocking(wf_solver* h, int pres_k, int vel_k);
+/* Which kernels run the Jacobi loops (no counterpart in the reference).
+ * WF_LOOPS_AUTO (default): a loop whose grid fits the GPU's registers and
+ * shared memories runs as one cooperative launch that keeps it there, any
+ * other as passes over memory.  WF_LOOPS_PASSES: passes always; an explicit
+ * depth or tile (wf_set_blocking, wf_set_tiles) selects it too.  Results do
+ * not depend on the mode.  Drops the handle's captured step graphs; rebuild
+ * batches that contain the handle afterwards. */
+enum { WF_LOOPS_AUTO = 0, WF_LOOPS_PASSES = 1 };
+int wf_set_loops(wf_solver* h, int mode);
 int wf_get_blocking(const wf_solver* h, int* pres_k, int* vel_k);
 /* Tile shapes of the Jacobi kernels: rows of the pressure multi-sweep tile
  * (32: 32 x 32 tiles, one block per SM; 16: 32 x 16 tiles, two blocks per

@@ -1,0 +1,90 @@
+"""Loops that keep the grid on chip against the pass kernels.
+
+Both run the same arithmetic in the same order on the same values, so every
+field must agree bit for bit: grids of one box and of many, boxes that
+overhang the domain on every axis, every count of cells a thread owns, odd
+extents, few sweeps, passes that also write iterate n - 1, the stretched mesh
+and the adjoint's kept iterates."""
+import numpy as np
+import pytest
+
+from unitywindsimulation_b200 import FvmSolverCuda, _lib, cases
+from unitywindsimulation_b200.adjoint import AdjointSolver
+
+from helpers import ALL_FIELDS
+
+pytestmark = pytest.mark.gpu
+
+
+def _pair(case):
+    out = []
+    for mode in (_lib.LOOPS_AUTO, _lib.LOOPS_PASSES):
+        s = FvmSolverCuda(case.cfg)
+        s.set_loops(mode)
+        cases.apply_case(s, case)
+        out.append(s)
+    return out
+
+
+def _same(a, b):
+    for f in ALL_FIELDS:
+        assert np.array_equal(a.get_field(f), b.get_field(f)), _lib.FIELD_NAMES[f]
+
+
+# extents chosen for 2, 3, 4, 6, 8, 10, 12, 14 and 16 cells a thread on 148
+# multiprocessors, with ragged last boxes
+GRIDS = [(24, 12, 16), (53, 31, 37), (12, 9, 13), (72, 40, 72), (88, 41, 77), (100, 50, 75), (104, 50, 97),
+         (103, 53, 104), (126, 63, 95), (130, 61, 110), (149, 61, 103)]
+
+
+@pytest.mark.parametrize("grid", GRIDS, ids=lambda g: "%dx%dx%d" % g)
+def test_steps_bit_identical(built, grid):
+    nx, ny, nz = grid
+    case = cases.small_case(nx=nx, ny=ny, nz=nz, seed=nx, nv=5, np_=7, les=nx % 2 == 0)
+    a, b = _pair(case)
+    for s in (a, b):
+        s.Step(2)
+    _same(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 8])
+def test_loops_outside_a_step(built, n):
+    """The operations also leave iterate n - 1, and start from the last iterate."""
+    case = cases.small_case(nx=45, ny=22, nz=31, seed=3)
+    a, b = _pair(case)
+    for s in (a, b):
+        s.Step(1)
+        s.op("vel_precompute"); s.op("vel_sweeps", n); s.op("pres_precompute")
+        s.op("pres_sweeps", n); s.op("pres_sweeps", n + 1)
+    _same(a, b)
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(log_inflow=True, les=True), dict(nx=15, x_split=(7, 4))],
+                         ids=["tunnel", "urban_les", "odd"])
+def test_stretched_mesh_bit_identical(built, kw):
+    a, b = _pair(cases.small_nonuniform_case(**kw))
+    for s in (a, b):
+        s.Step(3)
+        s.op("pres_sweeps", 4)
+    _same(a, b)
+    assert np.array_equal(a.get_face_flux(), b.get_face_flux())
+
+
+@pytest.mark.parametrize("grid", [(24, 12, 16), (41, 21, 30)], ids=lambda g: "%dx%dx%d" % g)
+def test_adjoint_iterates(built, grid):
+    """Recorded forward step bit for bit; the reversed step to the rounding
+    of its float atomics."""
+    case = cases.small_soft_case(*grid, nv=5, np_=6)
+    rng = np.random.default_rng(1)
+    n = case.n_cells
+    ub, pb = rng.standard_normal((3, n), dtype=np.float32), rng.standard_normal(n, dtype=np.float32)
+    got = []
+    for s in _pair(case):
+        s.Step(1)
+        with AdjointSolver(s) as adj:
+            got.append((adj.step_forward(), adj.step_vjp(ub, pb)))
+    (fa, va), (fb, vb) = got
+    for x, y in zip(fa, fb):
+        assert np.array_equal(x, y)
+    for x, y in ((va[0], vb[0]), (va[1], vb[1]), (va[3], vb[3])):
+        assert np.linalg.norm(x - y) <= 1e-5 * np.linalg.norm(y)

@@ -201,6 +201,7 @@ _SIGNATURES = {
     "wf_set_tiles": (c_int, [c_void_p, c_int, c_int, c_int, c_int]),
     "wf_get_tiles": (c_int, [c_void_p, POINTER(c_int), POINTER(c_int), POINTER(c_int), POINTER(c_int)]),
     "wf_set_blocking": (c_int, [c_void_p, c_int, c_int]),
+    "wf_set_loops": (c_int, [c_void_p, c_int]),
     "wf_get_blocking": (c_int, [c_void_p, POINTER(c_int), POINTER(c_int)]),
     "wf_export_open": (c_int, [c_void_p, c_char_p, c_int, c_int, c_int, POINTER(c_void_p)]),
     "wf_export_frame": (c_int, [c_void_p, c_float]),
@@ -225,6 +226,7 @@ PHASE_NAMES = ("les", "vel_pre", "vel_sweeps", "pres_pre", "pres_sweeps", "corre
 PHASE_COUNT = len(PHASE_NAMES)
 KERNEL_PRES_SWEEP = 0
 KERNEL_VEL_SWEEP = 1
+LOOPS_AUTO, LOOPS_PASSES = 0, 1
 
 _lib = None
 

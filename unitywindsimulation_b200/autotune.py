@@ -88,20 +88,26 @@ def tune_batch(batch, widths=(1, 2, 4, 0), steps: int = 2, modes=None) -> dict:
 
 def tune(solver, cache_path: str | None = DEFAULT_CACHE, reps: int = 5, device_name: str | None = None) -> dict:
     """Picks and applies the fastest blocking depths and tile shapes for
-    `solver`'s grid.  Returns {"pres_k", "pres_rows", "vel_k", "vel_block",
+    `solver`'s grid, and whether its loops run on chip.  Returns {"loops", "pres_k", "pres_rows", "vel_k", "vel_block",
     "pres_us_per_sweep", "vel_us_per_sweep", "cached"}."""
     name = device_name or _device_name()
     key = _key(solver, name)
     cache = load_cache(cache_path) if cache_path else {}
-    if key in cache and "pres_rows" in cache[key]:
+    if key in cache and "loops" in cache[key]:
         e = dict(cache[key])
         solver.set_blocking(e["pres_k"], e["vel_k"])
         solver.set_tiles(e["pres_rows"], tuple(e["vel_block"]))
+        solver.set_loops(e["loops"])
         e["cached"] = True
         return e
     saved = solver.get_blocking()
     _, vblk0 = solver.get_tiles()
     best_p, best_v = None, None
+    # the loop that keeps the grid on chip, where it fits (one launch is then
+    # the whole loop, more sweeps than any pass)
+    solver.set_loops(_lib.LOOPS_AUTO)
+    ms, _, sweeps = solver.time_kernel(_lib.KERNEL_PRES_SWEEP, reps=reps, flush_l2=True)
+    chip_us = ms * 1e3 / sweeps if sweeps > max(PRES_DEPTHS) else None
     for rows in PRES_ROWS:
         solver.set_tiles(rows, vblk0)
         for k in PRES_DEPTHS:
@@ -121,8 +127,11 @@ def tune(solver, cache_path: str | None = DEFAULT_CACHE, reps: int = 5, device_n
                 best_v = (k, blk, us)
     solver.set_blocking(best_p[0], best_v[0])
     solver.set_tiles(best_p[1], best_v[1])
-    e = {"pres_k": best_p[0], "pres_rows": best_p[1], "vel_k": best_v[0], "vel_block": list(best_v[1]),
-         "pres_us_per_sweep": best_p[2], "vel_us_per_sweep": best_v[2]}
+    on_chip = chip_us is not None and chip_us < best_p[2]
+    loops = _lib.LOOPS_AUTO if on_chip else _lib.LOOPS_PASSES
+    solver.set_loops(loops)
+    e = {"loops": loops, "pres_k": best_p[0], "pres_rows": best_p[1], "vel_k": best_v[0], "vel_block": list(best_v[1]),
+         "pres_us_per_sweep": chip_us if on_chip else best_p[2], "vel_us_per_sweep": best_v[2]}
     if cache_path:
         cache[key] = e
         save_cache(cache_path, cache)

@@ -873,6 +873,7 @@ struct wf_adjoint {
     float* gb = nullptr;     // adjoint of the 6 boundary planes (same layout)
     float* dragb = nullptr;  // adjoint of the drag field (N)
     double* dJ = nullptr;    // device accumulator of the objective
+    wf::Resident res;        // the solver's loop plans with a workspace of this handle's stream
     std::vector<float*> ck;  // stored states (4N each: u then p)
     std::string err;
 };
@@ -901,8 +902,11 @@ int adj_check_waits(wf_adjoint* a) {
     volatile int* st = a->h->hstat;
     if (!st || !*st) return WF_OK;
     *st = 0;
-    return adj_fail(a, WF_ERR_TIMEOUT, "a bounded wait of the TMA-staged pressure pass ran out; results are not valid");
+    return adj_fail(a, WF_ERR_TIMEOUT, "a bounded wait of a pressure loop's kernel ran out; results are not valid");
 }
+
+// On-chip pressure loops, or nullptr where the solver runs the pass kernels.
+const wf::Resident* adj_resident(const wf_adjoint* a) { return a->h->resident && a->h->dstat ? &a->res : nullptr; }
 
 float* V(const wf_adjoint* a, float* base, int k) { return base + (size_t)k * 3 * a->N; }
 float* S(const wf_adjoint* a, float* base, int k) { return base + (size_t)k * a->N; }
@@ -986,7 +990,7 @@ int record_step(wf_adjoint* a, Tape& t, const float* u_in, const float* p_in, in
         wf::launch_pres_coef_ptr(P, st, h->fl, t.D, t.iD, t.c3);
         wf::launch_inv_ptr(P, st, h->fl, t.Dp, t.ainv);
         WFA_CUDA(cudaMemsetAsync(t.qit, 0, s, st));
-        wf::launch_pres_stack(P, st, h->num_sms, t.c3, t.ainv, t.bp, t.qit, a->nP, true, tma_status(h));
+        wf::launch_pres_stack(P, st, h->num_sms, t.c3, t.ainv, t.bp, t.qit, a->nP, true, tma_status(h), adj_resident(a));
         const float* q = S(a, t.qit, a->nP);
         WFA_CUDA(cudaMemsetAsync(t.cbuf, 0, v, st));
         wf::launch_apply_vel(P, st, h->fl, q, t.D, t.iD, V(a, t.cbuf, 0), t.uout);
@@ -1000,7 +1004,7 @@ int record_step(wf_adjoint* a, Tape& t, const float* u_in, const float* p_in, in
             wf::launch_piso_aodu(P, st, h->fl, V(a, t.cbuf, m), t.uT, h->eddy, h->face, V(a, t.aod, m));
             wf::launch_piso_pre_ptr(P, st, h->fl, t.D, t.iD, V(a, t.aod, m), S(a, t.pai, m), S(a, t.prhs, m));
             wf::launch_pres_stack(P, st, h->num_sms, t.c3, S(a, t.pai, m), S(a, t.prhs, m), SIT(a, t, m, 0),
-                                  a->nP, true, tma_status(h));
+                                  a->nP, true, tma_status(h), adj_resident(a));
             const float* ss = SIT(a, t, m, a->nP);
             wf::launch_apply_pres(P, st, h->fl, ss, t.pout);
             wf::launch_piso_vel(P, st, h->fl, ss, t.D, t.iD, V(a, t.aod, m), V(a, t.cbuf, m + 1), t.uout);
@@ -1026,7 +1030,8 @@ void reverse_pres_loop(wf_adjoint* a, const float* ai, const float* c3, const fl
     }
     // slot j of a->Wp holds W^{n-j}
     wf::k_adj_pinit<<<wf::lin_blocks(a->N), 256, 0, st>>>((int)a->N, ai, a->sb, a->Wp);
-    if (n > 1) wf::launch_pres_stack(P, st, a->h->num_sms, c3, ai, nullptr, a->Wp, n - 1, false, tma_status(a->h));
+    if (n > 1) wf::launch_pres_stack(P, st, a->h->num_sms, c3, ai, nullptr, a->Wp, n - 1, false, tma_status(a->h),
+                                     adj_resident(a));
     if (wf::quad_ok(P, {ai, a->Wp, sstack, a->rb, a->dgb, a->c3b})) {
         const dim3 b4 = wf::cblk(), g4q((P.nx / 4 + b4.x - 1) / b4.x, (P.ny + b4.y - 1) / b4.y, (P.nz + b4.z - 1) / b4.z);
         wf::k_adj_pacc4<<<g4q, b4, 0, st>>>(P, n, ai, a->Wp, sstack, a->rb, a->dgb, a->c3b);
@@ -1119,6 +1124,7 @@ void free_adj(wf_adjoint* a) {
     a->blocks.clear();
     a->tapes.clear();
     if (a->dJ) cudaFree(a->dJ);
+    wf::resident_free(&a->res);
     for (float* p : a->ck)
         if (p) cudaFree(p);
     a->ck.clear();
@@ -1160,6 +1166,10 @@ int wf_adj_create(wf_solver* h, wf_adjoint** out) {
     al(&a->dragb, s);
     if (ok) ok = cudaMalloc((void**)&a->dJ, sizeof(double)) == cudaSuccess;
     if (ok) ok = ensure_tapes(a, 1) == WF_OK;
+    if (ok) {
+        a->res.pres = h->res.pres;
+        wf::resident_alloc(&a->res, a->st);
+    }
     if (ok) ok = cudaStreamSynchronize(a->st) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();

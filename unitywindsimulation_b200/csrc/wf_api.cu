@@ -118,6 +118,7 @@ void free_all(wf_solver* h) {
                     h->dbad, h->stage, h->bnd[0], h->drag, h->nbm, h->fpos, h->flux, h->nucoef};
     for (void* p : ptrs)
         if (p) cudaFree(p);
+    wf::resident_free(&h->res);
     if (h->hsum) cudaFreeHost(h->hsum);
     if (h->hstat) cudaFreeHost(h->hstat);
     if (h->cst) {
@@ -142,7 +143,7 @@ int sync(wf_solver* h) {
     if (h->hstat && *(volatile int*)h->hstat) {
         *(volatile int*)h->hstat = 0;
         return set_err(h, WF_ERR_TIMEOUT,
-                       "a bounded wait of the TMA-staged pressure sweep ran out; the pressure fields are not valid");
+                       "a bounded wait of a Jacobi loop's kernel ran out; the fields are not valid");
     }
     return WF_OK;
 }
@@ -265,6 +266,18 @@ int do_pres_sweeps(wf_solver* h, int n, bool allow_fast) {
     if (allow_fast && h->fast && !resid && n > 0 && !h->nonuniform) {
         WF_TRY(wf::pres_sweeps_fast(h, n, /*piso=*/false));
         return WF_OK;
+    }
+    if (allow_fast && h->fast && !resid && h->nonuniform && n >= 2 && wf::loops_on_chip(h, h->res.nupres)) {
+        // one launch; the output is another buffer than the input, the third
+        // one holds iterate n - 1 (only written outside a step)
+        const int in = h->pc_zero ? -1 : h->iPCL, out = in == 0 ? 1 : 0, prev = in < 0 ? 1 : 3 - in - out;
+        if (wf::launch_res_nupres(P, h->st, h->res.nupres, h->res.work, h->nucoef, h->bp, in < 0 ? nullptr : h->pcb[in],
+                                  h->pcb[out], h->in_step ? nullptr : h->pcb[prev], n, h->dstat) == cudaSuccess) {
+            h->pc_zero = false;
+            h->iPC = out;
+            h->iPCL = prev;
+            return WF_OK;
+        }
     }
     for (int k = 0; k < n; ++k) {
         const float* src = h->pc_zero ? nullptr : h->pcb[h->iPCL];
@@ -478,8 +491,9 @@ int run_step_eager(wf_solver* h) {
 
 int ensure_step_graph(wf_solver* h, const wf_solver::GraphEntry** out) {
     const auto key = role_key(h);
-    auto it = h->graphs.find(key);
-    if (it == h->graphs.end()) {
+    auto& graphs = h->in_batch ? h->batch_graphs : h->graphs;
+    auto it = graphs.find(key);
+    if (it == graphs.end()) {
         cudaGraph_t g = nullptr;
         WF_CUDA(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
         const int64_t step0 = h->step;
@@ -506,13 +520,13 @@ int ensure_step_graph(wf_solver* h, const wf_solver::GraphEntry** out) {
         ent.graph = g;
         ent.kernels = nk;
         ent.after = after;
-        e = cudaGraphInstantiate(&ent.exec, g, 0);
+        if (!h->in_batch) e = cudaGraphInstantiate(&ent.exec, g, 0);  // a batch clones the graph into its own
         if (e != cudaSuccess) {
             cudaGraphDestroy(g);
             h->err = std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e);
             return WF_ERR_CUDA;
         }
-        it = h->graphs.emplace(key, ent).first;
+        it = graphs.emplace(key, ent).first;
     }
     *out = &it->second;
     return WF_OK;
@@ -570,11 +584,13 @@ void commit_graph_step(wf_solver* h, const wf_solver::GraphEntry& e) {
 }
 
 void drop_graphs(wf_solver* h) {
-    for (auto& kv : h->graphs) {
-        if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
-        if (kv.second.graph) cudaGraphDestroy(kv.second.graph);
+    for (auto* m : {&h->graphs, &h->batch_graphs}) {
+        for (auto& kv : *m) {
+            if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
+            if (kv.second.graph) cudaGraphDestroy(kv.second.graph);
+        }
+        m->clear();
     }
-    h->graphs.clear();
 }
 
 }  // namespace wf
@@ -655,6 +671,10 @@ int wf_create(const wf_config* cfg, int device, wf_solver** out) {
     if (const char* v4 = std::getenv("WF_VEC4")) h->vec4 = std::atoi(v4);
     if (const char* pd = std::getenv("WF_PDL")) h->pdl = std::atoi(pd);
     if (const char* tm = std::getenv("WF_TMA")) h->pres_tma = std::atoi(tm);
+    // each of these names a form of the pass kernels, so it selects the passes
+    for (const char* v : {"WF_PRES_K", "WF_VEL_K", "WF_VEC4", "WF_PDL", "WF_TMA"})
+        if (std::getenv(v)) h->resident = 0;
+    if (const char* rs = std::getenv("WF_RESIDENT")) h->resident = std::atoi(rs) != 0;
 
     Params& P = h->P;
     P.nx = cfg->nx; P.ny = cfg->ny; P.nz = cfg->nz;
@@ -718,6 +738,9 @@ int wf_create(const wf_config* cfg, int device, wf_solver** out) {
     if (cudaHostAlloc((void**)&h->hstat, sizeof(int), cudaHostAllocMapped) != cudaSuccess) return fail(WF_ERR_OOM);
     *h->hstat = 0;
     if (cudaHostGetDevicePointer((void**)&h->dstat, h->hstat, 0) != cudaSuccess) return fail(WF_ERR_CUDA);
+    wf::resident_plan(P, h->num_sms, &h->res);
+    if (wf::resident_setup(h->res) != WF_OK) return fail(WF_ERR_CUDA);
+    wf::resident_alloc(&h->res, h->st);
 
     // Constructor sequence, FvmSolverGpu.cs:207-221.  Flags start all fluid
     // (zeroed allocation = CELL_FLUID); faceEddyVis starts at 0 because

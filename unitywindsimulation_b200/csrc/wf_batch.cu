@@ -442,7 +442,9 @@ int ensure_batch_graph(wf_batch* b, const wf_batch::Entry** out) {
         for (size_t i = 0; i < b->s.size(); ++i) {
             wf_solver* h = b->s[i];
             const wf_solver::GraphEntry* ge = nullptr;
+            h->in_batch = b->s.size() > 1;
             const int st = wf::ensure_step_graph(h, &ge);
+            h->in_batch = false;
             if (st != WF_OK) {
                 cudaGraphDestroy(parent);
                 return fail(b, st, "capturing a case's step failed: " + h->err);
@@ -528,7 +530,9 @@ int wf_batch_step(wf_batch* b, int n_steps) {
         if (!h->cfg.use_graph || h->cfg.calc_residual)
             return fail(b, WF_ERR_UNSUPPORTED, "batched cases need use_graph and no residual checks");
         if (!wf::step_graphable(h) && n_steps > 0) {
+            h->in_batch = b->s.size() > 1;
             const int st = wf::run_step_eager(h);
+            h->in_batch = false;
             if (st != WF_OK) return fail(b, st, "eager step failed: " + h->err);
             any_eager = true;
         }
@@ -711,6 +715,20 @@ int wf_set_blocking(wf_solver* h, int pres_k, int vel_k) {
     wf::drop_graphs(h);  // captured steps encode the old depths
     h->pres_k = pres_k;
     h->vel_k = vel_k;
+    h->resident = 0;  // an explicit depth selects the pass kernels
+    return WF_OK;
+}
+
+int wf_set_loops(wf_solver* h, int mode) {
+    if (!h) return WF_ERR_INVALID_ARG;
+    if (mode != WF_LOOPS_AUTO && mode != WF_LOOPS_PASSES) {
+        h->err = "mode must be WF_LOOPS_AUTO or WF_LOOPS_PASSES";
+        return WF_ERR_INVALID_ARG;
+    }
+    if (cudaSetDevice(h->device) != cudaSuccess) return WF_ERR_CUDA;
+    cudaStreamSynchronize(h->st);
+    wf::drop_graphs(h);  // captured steps encode the old loops
+    h->resident = mode == WF_LOOPS_AUTO;
     return WF_OK;
 }
 
@@ -728,6 +746,7 @@ int wf_set_tiles(wf_solver* h, int pres_rows, int vel_bx, int vel_by, int vel_bz
     h->vel_blk[0] = vel_bx;
     h->vel_blk[1] = vel_by;
     h->vel_blk[2] = vel_bz;
+    h->resident = 0;  // an explicit tile selects the pass kernels
     return WF_OK;
 }
 

@@ -1,0 +1,59 @@
+// wf_resident.cuh - Jacobi loops that keep the whole grid on chip
+// (wf_resident.cu): plan, workspace and launchers.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "wf_common.cuh"
+
+namespace wf {
+
+// Split of a grid into px x py x pz boxes of bx x by x bz cells, one box per
+// block and at most one block per multiprocessor.  bz is the number of cells
+// a thread owns (a z column); bz == 0: the grid does not fit on chip.
+struct ResPlan {
+    int bx = 0, by = 0, bz = 0, px = 0, py = 0, pz = 0;
+    int boxes() const { return px * py * pz; }
+};
+
+// Device workspace of the loops of one stream: the halo packets of both
+// parities and the epoch words.  One loop at a time may use it.
+struct ResWork {
+    void* pk = nullptr;
+    unsigned* ctl = nullptr;
+};
+
+// The plans of one handle's loops and their workspace.
+struct Resident {
+    ResPlan pres;      // uniform pressure loops
+    ResPlan nupres;    // non-uniform pressure loop
+    ResWork work;
+    bool ok(const ResPlan& p) const { return p.bz > 0 && work.pk != nullptr; }
+};
+
+// Plans for the grid of P on a device of `sms` multiprocessors.
+void resident_plan(const Params& P, int sms, Resident* r);
+// Attributes of the plans' kernels; call on the device before the first
+// launch.
+int resident_setup(const Resident& r);
+// Allocates / frees the workspace the plans need (stream-ordered zeroing on
+// st).  Without memory the plans stay unused: the loops run as passes.
+void resident_alloc(Resident* r, cudaStream_t st);
+void resident_free(Resident* r);
+
+// n >= 2 sweeps p = ainv (rhs - C p) of the uniform grid's pressure
+// equations in one cooperative launch, from pin (nullptr: zero), with the
+// iterates of k_pres_msweep / k_pres_tma4 bit for bit.  pout receives iterate
+// n on fluid cells, pprev (nullable) iterate n - 1; stack (nullable) every
+// iterate k = 1..n of every cell at stack + k N.  rhs nullptr: 0.  A bounded
+// wait that runs out sets *status to 1.
+cudaError_t launch_res_pres(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w, const float* c3,
+                            const float* ainv, const float* rhs, const float* pin, float* pout, float* pprev,
+                            float* stack, int n, int* status);
+// The same for the non-uniform grid: six face coefficients and 1/Dp
+// (coef, kNuCoefPlanes planes), right-hand side bp; the iterates of
+// k_nu_pres_sweep bit for bit.
+cudaError_t launch_res_nupres(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w,
+                              const float* coef, const float* bp, const float* pin, float* pout, float* pprev, int n,
+                              int* status);
+
+}  // namespace wf

@@ -7,6 +7,7 @@
 #include <tuple>
 
 #include "wf_common.cuh"
+#include "wf_resident.cuh"
 
 namespace wf {
 struct LoopRecorder;
@@ -97,6 +98,11 @@ struct wf_solver {
     // host word (hstat) and its device alias (dstat); nonzero = a wait ran out
     int* hstat = nullptr;
     int* dstat = nullptr;
+    // loops that keep the whole grid on chip (wf_resident.cu) where it fits;
+    // 0: the pass kernels (wf_set_loops, an explicit depth or tile, WF_RESIDENT=0)
+    int resident = 1;
+    wf::Resident res;
+    bool in_batch = false;    // the step being enqueued runs beside other cases' steps
     int vel_blk[3] = {32, 4, 2};  // block of the four-cell momentum sweep (256 threads)
     int num_sms = 148;        // multiprocessors of the device
     int pdl = 1;              // programmatic dependent launch in the non-uniform grid's sweep chains
@@ -117,9 +123,20 @@ struct wf_solver {
         long long kernels = 0;
     };
     std::map<RoleKey, GraphEntry> graphs;
+    std::map<RoleKey, GraphEntry> batch_graphs;  // the same for steps beside other cases (exec unused)
 };
 
 namespace wf {
+// Cells from which a case of a batch runs its loops on chip.  Such a loop
+// takes the whole GPU, so the cases' loops run one after another; passes of
+// small cases fill the GPU together.  Measured per batched step: 16 cases of
+// 0.06-0.21 M cells 3.37 ms in passes, 3.77 ms on chip; 16 cases of 0.7-1.75 M
+// cells 20.6 ms in passes, 19.4 ms with the ones that fit on chip.
+constexpr int kBatchOnChipCells = 500000;
+inline bool loops_on_chip(const wf_solver* h, const ResPlan& p) {
+    return h->resident && h->dstat && h->res.ok(p) && (!h->in_batch || h->P.N >= kBatchOnChipCells);
+}
+
 // Step-graph plumbing shared by the single-handle and the batched step.
 bool step_graphable(const wf_solver* h);
 // Captures (once per buffer-role assignment) the graph of one step from the

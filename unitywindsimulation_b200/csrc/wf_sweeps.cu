@@ -1062,6 +1062,19 @@ int record_pres_loop(wf_solver* h, int n, const float* rhs) {
 int pres_sweeps_fast(wf_solver* h, int n, bool piso) {
     const float* rhs = pres_coef(h, piso);
     if (h->rec) return record_pres_loop(h, n, rhs);
+    if (n >= 2 && loops_on_chip(h, h->res.pres)) {
+        // the whole loop on chip: output and iterate n - 1 go to the two
+        // buffers that are not the input
+        const int in = h->pc_zero ? -1 : h->iPCL, out = in == 0 ? 1 : 0, prev = in < 0 ? 1 : 3 - in - out;
+        if (launch_res_pres(h->P, h->st, h->res.pres, h->res.work, h->pcoef, h->pcoef + 3 * (size_t)h->P.N, rhs,
+                            in < 0 ? nullptr : h->pcb[in], h->pcb[out], h->in_step ? nullptr : h->pcb[prev], nullptr,
+                            n, h->dstat) == cudaSuccess) {
+            h->pc_zero = false;
+            h->iPC = out;
+            h->iPCL = prev;
+            return WF_OK;
+        }
+    }
     const int kmax = std::min(std::max(h->pres_k, 1), 4);
     if (kmax == 1) {
         for (int k = 0; k < n; ++k) {
@@ -1138,7 +1151,10 @@ int time_kernel(wf_solver* h, int which, int reps, bool flush, float* ms, double
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     float total = 0.f;
-    const int kv = std::min(std::max(h->vel_k, 1), 2), kp = std::min(std::max(h->pres_k, 1), 4);
+    // where the pressure loops run on chip one launch is a whole loop
+    const bool res_p = which == WF_KERNEL_PRES_SWEEP && loops_on_chip(h, h->res.pres) && h->cfg.pres_iters >= 2;
+    const int kv = std::min(std::max(h->vel_k, 1), 2);
+    const int kp = res_p ? h->cfg.pres_iters : std::min(std::max(h->pres_k, 1), 4);
     for (int r = 0; r < reps; ++r) {
         if (flush) k_flush_read<<<148 * 4, 512, 0, h->st>>>((const float4*)fbuf, flush_bytes / 16, (float*)fbuf);
         cudaEventRecord(e0, h->st);
@@ -1146,7 +1162,10 @@ int time_kernel(wf_solver* h, int which, int reps, bool flush, float* ms, double
             if (kv > 1) launch_vmsweep(h, kv, a, b, nullptr);
             else launch_vel_sweep_fast(h, a, b);
         } else {
-            if (kp > 1) launch_msweep(h, kp, rhs, a, b, nullptr);
+            if (res_p)
+                launch_res_pres(P, h->st, h->res.pres, h->res.work, h->pcoef, h->pcoef + 3 * N, rhs, a, b, nullptr,
+                                nullptr, kp, h->dstat);
+            else if (kp > 1) launch_msweep(h, kp, rhs, a, b, nullptr);
             else launch_pres_sweep_fast(h, rhs, a, b);
         }
         cudaEventRecord(e1, h->st);
@@ -1187,8 +1206,12 @@ void launch_stack_pass(const Params& P, cudaStream_t st, int sms, const float* c
         P, c3, ainv, rhs, in, nullptr, nullptr, zchunk, slots);
 }
 void launch_pres_stack(const Params& P, cudaStream_t st, int sms, const float* c3, const float* ainv,
-                       const float* rhs, float* stack, int n, bool from_zero, int* status) {
+                       const float* rhs, float* stack, int n, bool from_zero, int* status, const Resident* res) {
     const size_t N = P.N;
+    if (res && n >= 2 && res->ok(res->pres) &&
+        launch_res_pres(P, st, res->pres, res->work, c3, ainv, rhs, from_zero ? nullptr : stack, nullptr, nullptr,
+                        stack, n, status) == cudaSuccess)
+        return;
     for (int base = 0; base < n;) {
         const int k = std::min(4, n - base);
         const float* in = (base == 0 && from_zero) ? nullptr : stack + base * N;

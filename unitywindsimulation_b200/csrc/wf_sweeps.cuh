@@ -41,8 +41,11 @@ void launch_piso_pre_ptr(const Params& P, cudaStream_t st, const uint8_t* fl, co
 // first pass reads slot 0, or the all-zero iterate when from_zero is set.
 // Four-sweep passes take the TMA-staged kernel where it applies and
 // `status` is given (the handle's wait status), else k_pres_msweep<4, 32>.
+// res (nullable): plan and workspace of the on-chip loop, which then runs
+// all n sweeps in one launch where the grid fits.
 void launch_pres_stack(const Params& P, cudaStream_t st, int sms, const float* c3, const float* ainv,
-                       const float* rhs, float* stack, int n, bool from_zero, int* status = nullptr);
+                       const float* rhs, float* stack, int n, bool from_zero, int* status = nullptr,
+                       const Resident* res = nullptr);
 
 // ---- loop recording and persistent multi-case loops (wf_batch.cu) ----
 //

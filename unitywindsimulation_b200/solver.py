@@ -282,6 +282,11 @@ class FvmSolverCuda:
     def set_blocking(self, pres_k: int, vel_k: int) -> None:
         self._check(self._lib.wf_set_blocking(self._h, int(pres_k), int(vel_k)))
 
+    def set_loops(self, mode: int) -> None:
+        """_lib.LOOPS_AUTO (loops whose grid fits on chip run as one launch,
+        the default) or _lib.LOOPS_PASSES (wf_set_loops)."""
+        self._check(self._lib.wf_set_loops(self._h, int(mode)))
+
     def get_blocking(self):
         p, v = c_int(0), c_int(0)
         self._check(self._lib.wf_get_blocking(self._h, byref(p), byref(v)))
