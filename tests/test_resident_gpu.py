@@ -88,3 +88,37 @@ def test_adjoint_iterates(built, grid):
         assert np.array_equal(x, y)
     for x, y in ((va[0], vb[0]), (va[1], vb[1]), (va[3], vb[3])):
         assert np.linalg.norm(x - y) <= 1e-5 * np.linalg.norm(y)
+
+
+def test_loops_of_several_handles_at_once(built):
+    """Handles stepped side by side on their own streams (each loop is one
+    cooperative launch of up to every multiprocessor) and from their own
+    threads: the fields of stepping them one after another."""
+    import threading
+    grids = [(24, 12, 16), (64, 32, 48), (53, 31, 37), (104, 50, 97), (72, 40, 72), (48, 20, 28)]
+    cs = [cases.small_case(nx=x, ny=y, nz=z, seed=x, nv=4, np_=20) for x, y, z in grids]
+    got = []
+    for together in (False, True):
+        solvers = [FvmSolverCuda(c.cfg) for c in cs]
+        for s, c in zip(solvers, cs):
+            cases.apply_case(s, c)
+            s.Step(1)
+        if together:
+            for _ in range(6):
+                for s in solvers:
+                    s.step_async(1)
+            threads = [threading.Thread(target=s.Step, args=(4,)) for s in solvers]
+            for t in threads:
+                t.start()
+            for t in threads:
+                t.join()
+        else:
+            for s in solvers:
+                s.Step(10)
+        for s in solvers:
+            s.sync()
+        got.append([(s.GetVelField(), s.GetPresField()) for s in solvers])
+        for s in solvers:
+            s.close()
+    for (va, pa), (vb, pb) in zip(*got):
+        assert np.array_equal(va, vb) and np.array_equal(pa, pb)

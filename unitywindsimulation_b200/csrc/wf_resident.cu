@@ -25,7 +25,9 @@
 // steps, with the four-sweep passes before: 623 -> 310 us (64 x 32 x 48, PISO,
 // 90 pressure sweeps), 5077 -> 1467 us (80 x 40 x 40, 1000), 2425 -> 1059 us (100 x 50 x
 // 100, 400), 1278 -> 1027 us (128 x 64 x 96, 90), 1396 -> 1186 us (149 x 61 x 103, 90),
-// 9761 -> 8258 us (100 x 50 x 100 stretched mesh, 2000).
+// 9761 -> 8258 us (100 x 50 x 100 stretched mesh, 2000).  With the momentum loop
+// on chip too: 310 -> 269 us (64 x 32 x 48, 50 sweeps), 1467 -> 1399 us (80 x 40 x 40,
+// 100), 1059 -> 982 us (100 x 50 x 100, 50), 8258 -> 6753 us (stretched mesh, 800).
 //
 // The launch is cooperative, so all blocks are resident and every packet
 // that is waited for will be sent.  The waits are bounded all the same
@@ -55,6 +57,25 @@ __device__ __forceinline__ void put(unsigned long long* p, float v, unsigned ep)
 __device__ __forceinline__ unsigned long long get(const unsigned long long* p) {
     unsigned long long w;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p));
+    return w;
+}
+
+// Three components and the epoch in one 128-bit packet (a scalar 128-bit
+// access is single-copy atomic as well).
+struct Packet3 {
+    unsigned long long lo, hi;   // x, y | z, epoch
+};
+__device__ __forceinline__ void put3(Packet3* p, float x, float y, float z, unsigned ep) {
+    const unsigned long long lo = ((unsigned long long)__float_as_uint(y) << 32) | __float_as_uint(x);
+    const unsigned long long hi = ((unsigned long long)ep << 32) | __float_as_uint(z);
+    asm volatile("{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], w;\n\t}" ::"l"(p),
+                 "l"(lo), "l"(hi));
+}
+__device__ __forceinline__ Packet3 get3(const Packet3* p) {
+    Packet3 w;
+    asm volatile("{\n\t.reg .b128 w;\n\tld.relaxed.gpu.global.b128 w, [%2];\n\tmov.b128 {%0, %1}, w;\n\t}"
+                 : "=l"(w.lo), "=l"(w.hi)
+                 : "l"(p));
     return w;
 }
 
@@ -432,9 +453,234 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
     epoch_end(a.ctl, base, (unsigned)a.n + 1u);
 }
 
+// ---------------------------------------------------------------- momentum
+// Sweeps u = (1/D) (sum_f A_f u_f + b) of the three components.  One shared
+// box (a second barrier a sweep separates its readers from its writers: two
+// boxes of three components leave no room for the rest).  Above kVelRegR cells
+// a thread b and the second and third component of 1/D live in shared memory.
+constexpr int kVelRegR = 4;
+constexpr size_t vel_smem(int R) {
+    return 3 * (size_t)plane_of(R) * R * sizeof(float) + (R > kVelRegR ? 5 * (size_t)R * NT * sizeof(float) : 0);
+}
+static_assert(vel_smem(8) <= kSmemMax, "box exceeds the shared memory of one block");
+
+struct VelArgs {
+    int nx, ny, nz, n;
+    ResPlan pl;
+    const float *A, *iD, *bv, *uin;
+    float *uout, *uprev;
+    Packet3* pk;
+    size_t half;
+    unsigned* ctl;
+    int* status;
+};
+
+// receive() for three components.
+template <int R, bool RIM>
+__device__ __forceinline__ bool receive3(const Links& l, int rim, float* v, const Packet3* pk, unsigned ep, float hu[3],
+                                         float hd[3]) {
+    const bool nu = l.ru >= 0, nd = l.rd >= 0, ne = RIM && l.re >= 0;
+    const Packet3 *pu = pk + (nu ? l.ru : 0), *pd = pk + (nd ? l.rd : 0), *pe = pk + (ne ? l.re : 0);
+    constexpr int PS = plane_of(R);
+    int left = kRounds;
+    bool ok;
+    if (RIM) {
+        // the edge cells first: they arrive last
+        constexpr int U = R <= 4 ? R : (R + 1) / 2;
+#pragma unroll
+        for (int r0 = 0; r0 < R; r0 += U) {
+            Packet3 w[U];
+            do {
+#pragma unroll
+                for (int q = 0; q < U; ++q) w[q] = get3(pe + (r0 + q < R ? r0 + q : R - 1) * rim);
+                ok = true;
+#pragma unroll
+                for (int q = 0; q < U; ++q) ok = ok && (unsigned)(w[q].hi >> 32) == ep;
+                ok = ok || !ne;
+            } while (!__all_sync(0xffffffffu, ok) && --left);
+            if (left == 0) return false;
+            if (ne) {
+#pragma unroll
+                for (int q = 0; q < U; ++q)
+                    if (r0 + q < R) {
+                        float* o = v + l.he + (r0 + q) * PS;
+                        o[0] = __uint_as_float((unsigned)w[q].lo);
+                        o[R * PS] = __uint_as_float((unsigned)(w[q].lo >> 32));
+                        o[2 * R * PS] = __uint_as_float((unsigned)w[q].hi);
+                    }
+            }
+        }
+    }
+    Packet3 wu, wd;
+    do {
+        wu = get3(pu);
+        wd = get3(pd);
+        ok = (!nu || (unsigned)(wu.hi >> 32) == ep) && (!nd || (unsigned)(wd.hi >> 32) == ep);
+    } while (!__all_sync(0xffffffffu, ok) && --left);
+    if (left == 0) return false;
+    hu[0] = nu ? __uint_as_float((unsigned)wu.lo) : 0.f;
+    hu[1] = nu ? __uint_as_float((unsigned)(wu.lo >> 32)) : 0.f;
+    hu[2] = nu ? __uint_as_float((unsigned)wu.hi) : 0.f;
+    hd[0] = nd ? __uint_as_float((unsigned)wd.lo) : 0.f;
+    hd[1] = nd ? __uint_as_float((unsigned)(wd.lo >> 32)) : 0.f;
+    hd[2] = nd ? __uint_as_float((unsigned)wd.hi) : 0.f;
+    return true;
+}
+
+template <int R>
+__global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelArgs a) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr bool kShared = R > kVelRegR;
+    constexpr int PS = plane_of(R), CS = R * PS;  // plane, component
+    const unsigned base = epoch_begin(a.ctl);
+    const Box b = make_box(a.pl);
+    float* priv = sm + 3 * CS;                    // [5][R][NT]: b, second and third component of 1/D
+    const int tid = threadIdx.x;
+    const int sxy = a.nx * a.ny;
+    const size_t N = (size_t)sxy * a.nz;
+    int lx, ly;
+    const bool own = column_of(b, a.pl, tid, lx, ly), rim = tid < b.inner0;
+    const int x = b.x0 + lx, y = b.y0 + ly;
+    const bool inxy = own && x < a.nx && y < a.ny;
+    const int i0 = inxy ? (b.z0 * a.ny + y) * a.nx + x : 0;
+    const int o0 = (ly + 1) * b.sx + lx + 1;
+    const Links l = make_links(b, a.pl, own);
+    // the input iterate with its halo, zero outside the domain
+    for (int o = tid; o < 3 * CS; o += NT) sm[o] = 0.f;
+    __syncthreads();
+    float u[3][R], hu[3] = {0.f, 0.f, 0.f}, hd[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            u[c][r] = inxy && b.z0 + r < a.nz ? __ldg(a.uin + c * N + i0 + r * sxy) : 0.f;
+            if (own) sm[c * CS + r * PS + o0] = u[c][r];
+        }
+        if (inxy && b.z0 > 0) hd[c] = __ldg(a.uin + c * N + i0 - sxy);
+        if (inxy && b.z0 + R < a.nz) hu[c] = __ldg(a.uin + c * N + i0 + R * sxy);
+    }
+    if (tid < b.rim + 4) {
+        const int hy = b.y0 + l.he / b.sx - 1, hx = b.x0 + l.he % b.sx - 1;
+        if (hx >= 0 && hx < a.nx && hy >= 0 && hy < a.ny)
+            for (int c = 0; c < 3; ++c)
+                for (int r = 0; r < R && b.z0 + r < a.nz; ++r)
+                    sm[c * CS + r * PS + l.he] = __ldg(a.uin + c * N + (size_t)(b.z0 + r) * sxy + hy * a.nx + hx);
+    }
+    // the column's coefficients (1/D is 0 on solid cells, whose b is not
+    // theirs)
+    float A[6][R], d0[R], d12[kShared ? 1 : 2][kShared ? 1 : R], bb[kShared ? 1 : 3][kShared ? 1 : R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = i0 + r * sxy;
+        const bool in = inxy && b.z0 + r < a.nz;
+#pragma unroll
+        for (int f = 0; f < 6; ++f) A[f][r] = in ? __ldg(a.A + f * N + i) : 0.f;
+        d0[r] = in ? __ldg(a.iD + i) : 0.f;
+        const bool fluid = d0[r] != 0.f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float v = fluid ? __ldg(a.bv + c * N + i) : 0.f;
+            if (kShared) priv[(c * R + r) * NT + tid] = v;
+            else bb[kShared ? 0 : c][kShared ? 0 : r] = v;
+            if (c > 0) {
+                const float d = fluid ? __ldg(a.iD + c * N + i) : 0.f;
+                if (kShared) priv[((2 + c) * R + r) * NT + tid] = d;
+                else d12[kShared ? 0 : c - 1][kShared ? 0 : r] = d;
+            }
+        }
+    }
+    float* cur = sm + o0;
+    // component c of cell r, in the order of k_vel_sweep4
+    auto cell = [&](int c, int r, float up, float below) {
+        const float* q = cur + c * CS + r * PS;
+        float acc = A[0][r] * q[1];
+        acc += A[1][r] * q[-1];
+        acc += A[2][r] * cur[b.sx + c * CS + r * PS];
+        acc += A[3][r] * (cur - b.sx)[c * CS + r * PS];
+        acc += A[4][r] * up;
+        acc += A[5][r] * below;
+        const float rhs = kShared ? priv[(c * R + r) * NT + tid] : bb[kShared ? 0 : c][kShared ? 0 : r];
+        const float d = c == 0 ? d0[r]
+                      : kShared ? priv[((2 + c) * R + r) * NT + tid] : d12[kShared ? 0 : (c > 0 ? c - 1 : 0)][kShared ? 0 : r];
+        return d * (acc + rhs);
+    };
+    float v0[3], vT[3];
+    auto ends = [&]() {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            v0[c] = cell(c, 0, u[c][1], hd[c]);
+            vT[c] = cell(c, R - 1, hu[c], u[c][R - 2]);
+        }
+    };
+    auto middle = [&]() {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            float below = u[c][0];
+            const float top = u[c][R - 1];
+#pragma unroll
+            for (int r = 1; r < R - 1; ++r) {
+                const float old = u[c][r];
+                u[c][r] = cell(c, r, r + 1 < R - 1 ? u[c][r + 1 < R ? r + 1 : 0] : top, below);
+                below = old;
+            }
+            u[c][0] = v0[c];
+            u[c][R - 1] = vT[c];
+        }
+    };
+    auto emit = [&](float* out) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (inxy && b.z0 + r < a.nz && d0[r] != 0.f) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) out[c * N + i0 + r * sxy] = u[c][r];
+            }
+    };
+    __syncthreads();
+    Packet3 *pk = a.pk, *pk_next = a.pk + a.half;
+    unsigned ep = base;
+    bool bad = false;
+    const bool has_halo = gridDim.x > 1 && (tid & ~31) < b.inner0 + inner_of(a.pl);
+    for (int k = 1; k < a.n; ++k) {
+        ++ep;
+        ends();
+        if (l.sd >= 0) put3(pk + l.sd, v0[0], v0[1], v0[2], ep);
+        if (l.su >= 0) put3(pk + l.su, vT[0], vT[1], vT[2], ep);
+        middle();
+        if (l.se >= 0) {
+            Packet3* dst = pk + l.se;
+#pragma unroll
+            for (int r = 0; r < R; ++r) put3(dst + r * b.rim, u[0][r], u[1][r], u[2][r], ep);
+        }
+        __syncthreads();
+        if (own) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int r = 0; r < R; ++r) cur[c * CS + r * PS] = u[c][r];
+        }
+        if (has_halo)
+            bad = rim ? !receive3<R, true>(l, b.rim, sm, pk, ep, hu, hd) : !receive3<R, false>(l, b.rim, sm, pk, ep, hu, hd);
+        if (__syncthreads_or(bad)) break;
+        Packet3* t = pk;
+        pk = pk_next;
+        pk_next = t;
+    }
+    if (ep != base + (unsigned)a.n - 1u || __syncthreads_or(bad)) bad = true;
+    if (bad) {
+        if (tid == 0 && a.status) atomicExch(a.status, 1);
+    } else {
+        if (a.uprev) emit(a.uprev);
+        ends();
+        middle();
+        emit(a.uout);
+    }
+    epoch_end(a.ctl, base, (unsigned)a.n + 1u);
+}
+
 // Cells per thread the kernels are built for.
 constexpr int kPresR[] = {2, 3, 4, 6, 8, 10, 12, 14, 16};
 constexpr int kNuPresR[] = {2, 3, 4, 6, 8};
+constexpr int kVelR[] = {2, 3, 4, 6, 8};
 
 using PresKernel = void (*)(const PresArgs);
 template <bool NU, bool STACK>
@@ -457,6 +703,18 @@ PresKernel pres_kernel(int R) {
         }
     }
     return nullptr;
+}
+
+using VelKernel = void (*)(const VelArgs);
+VelKernel vel_kernel(int R) {
+    switch (R) {
+        case 2: return k_res_vel<2>;
+        case 3: return k_res_vel<3>;
+        case 4: return k_res_vel<4>;
+        case 6: return k_res_vel<6>;
+        case 8: return k_res_vel<8>;
+        default: return nullptr;
+    }
 }
 
 // The split with the least estimated time of a sweep.  Measured (us a sweep):
@@ -515,7 +773,7 @@ cudaError_t launch_coop(const void* fn, int blocks, size_t smem, cudaStream_t st
 
 int resident_setup(const Resident& r) {
     cudaError_t e = cudaSuccess;
-    auto opt_in = [&](PresKernel k) {
+    auto opt_in = [&](auto k) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
     };
     if (r.pres.bz > 0) {
@@ -523,19 +781,23 @@ int resident_setup(const Resident& r) {
         opt_in(pres_kernel<false, true>(r.pres.bz));
     }
     if (r.nupres.bz > 0) opt_in(pres_kernel<true, false>(r.nupres.bz));
+    if (r.vel.bz > 0) opt_in(vel_kernel(r.vel.bz));
     return e == cudaSuccess ? WF_OK : WF_ERR_CUDA;
 }
 
 void resident_plan(const Params& P, int sms, Resident* r) {
     r->pres = make_plan(P, sms, kPresR);
     r->nupres = make_plan(P, sms, kNuPresR);
+    r->vel = make_plan(P, sms, kVelR);
 }
 
 void resident_alloc(Resident* r, cudaStream_t st) {
-    const size_t n = std::max(packets(r->pres), packets(r->nupres));
-    if (n == 0 || r->work.pk) return;
-    // the epoch words follow the packets
-    const size_t bytes = 2 * n * sizeof(unsigned long long) + 16;
+    // both parities of the pressure packets, then of the momentum packets
+    // (apart: a momentum packet's words must not be read as pressure
+    // packets), then the epoch words
+    const size_t np = 2 * std::max(packets(r->pres), packets(r->nupres)), nv = 2 * packets(r->vel);
+    if (np + nv == 0 || r->work.pk) return;
+    const size_t bytes = np * sizeof(unsigned long long) + nv * sizeof(Packet3) + 16;
     void* pk = nullptr;
     if (cudaMalloc(&pk, bytes) != cudaSuccess) {
         cudaGetLastError();
@@ -547,7 +809,8 @@ void resident_alloc(Resident* r, cudaStream_t st) {
         return;
     }
     r->work.pk = pk;
-    r->work.ctl = reinterpret_cast<unsigned*>(static_cast<unsigned long long*>(pk) + 2 * n);
+    r->work.pk3 = static_cast<unsigned long long*>(pk) + np;  // np is even: 16-byte aligned
+    r->work.ctl = reinterpret_cast<unsigned*>(static_cast<Packet3*>(r->work.pk3) + nv);
 }
 
 void resident_free(Resident* r) {
@@ -587,6 +850,24 @@ cudaError_t launch_res_nupres(const Params& P, cudaStream_t st, const ResPlan& p
                               const float* coef, const float* bp, const float* pin, float* pout, float* pprev, int n,
                               int* status) {
     return launch_pres<true>(P, st, pl, w, coef, coef + 6 * (size_t)P.N, bp, pin, pout, pprev, nullptr, n, status);
+}
+
+cudaError_t launch_res_vel(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w, const float* A,
+                           const float* iD, const float* bv, const float* uin, float* uout, float* uprev, int n,
+                           int* status) {
+    VelArgs a = {};
+    a.nx = P.nx; a.ny = P.ny; a.nz = P.nz; a.n = n;
+    a.pl = pl;
+    a.A = A; a.iD = iD; a.bv = bv; a.uin = uin;
+    a.uout = uout; a.uprev = uprev;
+    a.pk = static_cast<Packet3*>(w.pk3);
+    a.half = packets(pl);
+    a.ctl = w.ctl;
+    a.status = status;
+    const cudaError_t e = launch_coop((const void*)vel_kernel(pl.bz), pl.boxes(), vel_smem(pl.bz), st, &a);
+    if (e == cudaSuccess) WF_COUNT_LAUNCH();
+    else cudaGetLastError();
+    return e;
 }
 
 }  // namespace wf

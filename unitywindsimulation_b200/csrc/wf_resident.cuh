@@ -18,7 +18,8 @@ struct ResPlan {
 // Device workspace of the loops of one stream: the halo packets of both
 // parities and the epoch words.  One loop at a time may use it.
 struct ResWork {
-    void* pk = nullptr;
+    void* pk = nullptr;    // the allocation; 64-bit packets of the pressure loops
+    void* pk3 = nullptr;   // 128-bit packets of the momentum loop
     unsigned* ctl = nullptr;
 };
 
@@ -26,6 +27,7 @@ struct ResWork {
 struct Resident {
     ResPlan pres;      // uniform pressure loops
     ResPlan nupres;    // non-uniform pressure loop
+    ResPlan vel;       // momentum loop
     ResWork work;
     bool ok(const ResPlan& p) const { return p.bz > 0 && work.pk != nullptr; }
 };
@@ -55,5 +57,12 @@ cudaError_t launch_res_pres(const Params& P, cudaStream_t st, const ResPlan& pl,
 cudaError_t launch_res_nupres(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w,
                               const float* coef, const float* bp, const float* pin, float* pout, float* pprev, int n,
                               int* status);
+// n >= 2 momentum sweeps u = (1/D) (sum_f A_f u_f + b) from uin in one
+// launch: A holds A_E..A_D, iD the three components of 1/D.  The iterates of
+// k_vel_sweep4 bit for bit; uout (uprev, nullable) receives iterate n (n - 1)
+// on fluid cells and may not alias uin.
+cudaError_t launch_res_vel(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w, const float* A,
+                           const float* iD, const float* bv, const float* uin, float* uout, float* uprev, int n,
+                           int* status);
 
 }  // namespace wf

@@ -926,6 +926,22 @@ int record_vel_loop(wf_solver* h, int n) {
 int vel_sweeps_fast(wf_solver* h, int n) {
     vel_coef(h);
     if (h->rec) return record_vel_loop(h, n);
+    if (n >= 2 && loops_on_chip(h, h->res.vel)) {
+        // the whole loop on chip, into two buffers that are neither its input
+        // nor velFieldLastTime
+        const size_t N = h->P.N;
+        const int in = h->iter_alias ? h->iT : h->iI;
+        int out = 0, prev = 0;
+        while (out == h->iT || out == in) ++out;
+        while (prev == h->iT || prev == in || prev == out) ++prev;
+        if (launch_res_vel(h->P, h->st, h->res.vel, h->res.work, h->vcoef, h->vcoef + 6 * N, h->bv, h->vb[in],
+                           h->vb[out], h->in_step ? nullptr : h->vb[prev], n, h->dstat) == cudaSuccess) {
+            h->iF = out;
+            h->iI = prev;
+            h->iter_alias = false;
+            return WF_OK;
+        }
+    }
     const int kmax = std::min(std::max(h->vel_k, 1), 2);
     if (kmax > 1) {
         // Passes of up to kmax sweeps over buffers other than velFieldLastTime;
@@ -1153,13 +1169,17 @@ int time_kernel(wf_solver* h, int which, int reps, bool flush, float* ms, double
     float total = 0.f;
     // where the pressure loops run on chip one launch is a whole loop
     const bool res_p = which == WF_KERNEL_PRES_SWEEP && loops_on_chip(h, h->res.pres) && h->cfg.pres_iters >= 2;
-    const int kv = std::min(std::max(h->vel_k, 1), 2);
+    const bool res_v = which == WF_KERNEL_VEL_SWEEP && loops_on_chip(h, h->res.vel) && h->cfg.vel_iters >= 2;
+    const int kv = res_v ? h->cfg.vel_iters : std::min(std::max(h->vel_k, 1), 2);
     const int kp = res_p ? h->cfg.pres_iters : std::min(std::max(h->pres_k, 1), 4);
     for (int r = 0; r < reps; ++r) {
         if (flush) k_flush_read<<<148 * 4, 512, 0, h->st>>>((const float4*)fbuf, flush_bytes / 16, (float*)fbuf);
         cudaEventRecord(e0, h->st);
         if (which == WF_KERNEL_VEL_SWEEP) {
-            if (kv > 1) launch_vmsweep(h, kv, a, b, nullptr);
+            if (res_v)
+                launch_res_vel(P, h->st, h->res.vel, h->res.work, h->vcoef, h->vcoef + 6 * N, h->bv, a, b, nullptr, kv,
+                               h->dstat);
+            else if (kv > 1) launch_vmsweep(h, kv, a, b, nullptr);
             else launch_vel_sweep_fast(h, a, b);
         } else {
             if (res_p)
