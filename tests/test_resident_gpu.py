@@ -122,3 +122,57 @@ def test_loops_of_several_handles_at_once(built):
             s.close()
     for (va, pa), (vb, pb) in zip(*got):
         assert np.array_equal(va, vb) and np.array_equal(pa, pb)
+
+
+@pytest.mark.parametrize("tols", [(1e-15, 1e-15), (1e-15, None), (None, 1e-15)], ids=["never", "pressure", "momentum"])
+@pytest.mark.parametrize("stretched", [False, True], ids=["uniform", "stretched"])
+def test_residual_checks_between_fast_loops(built, tols, stretched):
+    """With residual checks the pressure loop runs on chip from check to
+    check; the sweep at which a tolerance ends a loop, the buffer roles the
+    reference's break leaves, the residuals and the fields are the oracle's
+    (whose loop checks sweep by sweep)."""
+    from helpers import REL_TOL, rel_l2
+    from oracle import OracleSolver
+    case = cases.small_nonuniform_case(nv=13, np_=23) if stretched else \
+        cases.small_case(nx=45, ny=22, nz=31, seed=2, piso=False, nv=13, np_=23)
+    case.cfg.calc_residual, case.cfg.vel_res_interval, case.cfg.pres_res_interval = 1, 4, 5
+    case.cfg.vel_tol = case.cfg.pres_tol = 1e-15
+    if None in tols:  # a tolerance between the residuals of two checked sweeps of the first step
+        o = OracleSolver(case.cfg, 32)
+        cases.apply_case(o, case)
+        o.op("vel_precompute")
+        name, sweeps = ("vel", 8) if tols[0] is None else ("pres", 10)
+        if name == "pres":
+            o.op("vel_sweeps", 13); o.op("pres_precompute")
+        o.op(name + "_sweeps", sweeps)
+        setattr(case.cfg, name + "_tol", 0.999 * o.op_residual(name))
+    got = []
+    for make in (FvmSolverCuda, lambda c: OracleSolver(c, 32)):
+        s = make(case.cfg)
+        cases.apply_case(s, case)
+        s.Step(1)
+        got.append((s, s.residuals()))
+    (g, rg), (o, ro) = got
+    # a residual is a difference of two iterates: each carries the rounding of
+    # its last sum of eight terms, so the norm is known to 8 eps of D u (Dp p')
+    rms = lambda a: float(np.sqrt(np.mean(np.square(a, dtype=np.float64))))  # noqa: E731
+    floors = [8 * 2.0 ** -24 * rms(o.get_field(d) * o.get_field(v))
+              for d, v in ((_lib.FIELD_D, _lib.FIELD_VEL), (_lib.FIELD_DP, _lib.FIELD_PRES_CORRECT))]
+    for a, b, floor in zip(rg, ro, floors):
+        assert abs(a - b) <= 1e-3 * abs(b) + floor
+    for f in (_lib.FIELD_VEL_LAST_TIME, _lib.FIELD_PRES):
+        assert rel_l2(g.get_field(f), o.get_field(f)) <= REL_TOL, _lib.FIELD_NAMES[f]
+
+
+@pytest.mark.parametrize("stretched", [False, True], ids=["uniform", "stretched"])
+def test_checked_steps_bit_identical(built, stretched):
+    """Residual checks: on chip between the checks against one sweep a launch."""
+    case = cases.small_nonuniform_case(nv=9, np_=23) if stretched else \
+        cases.small_case(nx=45, ny=22, nz=31, seed=2, piso=False, nv=9, np_=23)
+    case.cfg.calc_residual, case.cfg.vel_res_interval, case.cfg.pres_res_interval = 1, 4, 5
+    case.cfg.vel_tol = case.cfg.pres_tol = 1e-15
+    a, b = _pair(case)
+    for s in (a, b):
+        s.Step(2)
+    _same(a, b)
+    assert a.residuals() == b.residuals()

@@ -208,6 +208,23 @@ int read_residual(wf_solver* h, double* out) {
     return WF_OK;
 }
 
+// One step's residual check: sqrt(sum / terms) below the tolerance.
+int vel_converged(wf_solver* h, const float* u, const float* last, bool* done) {
+    wf::launch_vel_residual(h->P, h->st, h->Dv, u, last, h->part, h->dsum);
+    double s = 0.0;
+    WF_TRY(read_residual(h, &s));
+    h->res_vel = (float)std::sqrt(s / (3.0 * h->P.N));
+    *done = h->res_vel < h->cfg.vel_tol;
+    return WF_OK;
+}
+int pres_converged(wf_solver* h, const float* p, const float* last, bool* done) {
+    wf::launch_pres_residual(h->P, h->st, h->Dp, p, last, h->part, h->dsum);
+    double s = 0.0;
+    WF_TRY(read_residual(h, &s));
+    h->res_pres = (float)std::sqrt(s / double(h->P.N));
+    *done = h->res_pres < h->cfg.pres_tol;
+    return WF_OK;
+}
 // VelPredict loop (FvmSolverGpu.cs:1244-1279) with n sweeps.
 int do_vel_sweeps(wf_solver* h, int n, bool allow_fast) {
     const Params& P = h->P;
@@ -228,11 +245,9 @@ int do_vel_sweeps(wf_solver* h, int n, bool allow_fast) {
             wf::launch_vel_sweep(P, h->st, h->fl, src, h->vb[h->iT], h->eddy, h->face, h->Dv, h->bv, h->vb[h->iF]);
         WF_CHECK_LAUNCH();
         if (resid && k % h->cfg.vel_res_interval == 0) {
-            wf::launch_vel_residual(P, h->st, h->Dv, h->vb[h->iF], src, h->part, h->dsum);
-            double s = 0.0;
-            WF_TRY(read_residual(h, &s));
-            h->res_vel = (float)std::sqrt(s / (3.0 * P.N));
-            if (h->res_vel < h->cfg.vel_tol) break;
+            bool done = false;
+            WF_TRY(vel_converged(h, h->vb[h->iF], src, &done));
+            if (done) break;
         }
         std::swap(h->iI, h->iF);
         h->iter_alias = false;
@@ -263,22 +278,20 @@ int do_pres_precompute(wf_solver* h) {
 int do_pres_sweeps(wf_solver* h, int n, bool allow_fast) {
     const Params& P = h->P;
     const bool resid = h->cfg.calc_residual != 0;
-    if (allow_fast && h->fast && !resid && n > 0 && !h->nonuniform) {
+    allow_fast = allow_fast && h->fast;
+    if (allow_fast && !resid && n > 0 && !h->nonuniform) {
         WF_TRY(wf::pres_sweeps_fast(h, n, /*piso=*/false));
         return WF_OK;
     }
-    if (allow_fast && h->fast && !resid && h->nonuniform && n >= 2 && wf::loops_on_chip(h, h->res.nupres)) {
-        // one launch; the output is another buffer than the input, the third
-        // one holds iterate n - 1 (only written outside a step)
-        const int in = h->pc_zero ? -1 : h->iPCL, out = in == 0 ? 1 : 0, prev = in < 0 ? 1 : 3 - in - out;
-        if (wf::launch_res_nupres(P, h->st, h->res.nupres, h->res.work, h->nucoef, h->bp, in < 0 ? nullptr : h->pcb[in],
-                                  h->pcb[out], h->in_step ? nullptr : h->pcb[prev], n, h->dstat) == cudaSuccess) {
-            h->pc_zero = false;
-            h->iPC = out;
-            h->iPCL = prev;
-            return WF_OK;
-        }
-    }
+    if (allow_fast && !resid && n >= 2 && wf::loops_on_chip(h, h->res.nupres) &&
+        wf::pres_sweeps_on_chip(h, n, true, !h->in_step))
+        return WF_OK;
+    // with residual checks: the sweeps up to the next one on chip, in the
+    // sums of the kernels below.  One sweep a launch took 6.5 of the 8.2 ms of
+    // a step on 100 x 50 x 100 (400 sweeps, checked every 20).  (The momentum
+    // loop has no such form: 12 instead of 7 coefficients a cell do not fit.)
+    const bool chip = allow_fast && resid && wf::loops_on_chip(h, h->nonuniform ? h->res.nupres : h->res.pres);
+    bool coef_done = false;
     for (int k = 0; k < n; ++k) {
         const float* src = h->pc_zero ? nullptr : h->pcb[h->iPCL];
         if (h->nonuniform)
@@ -287,13 +300,18 @@ int do_pres_sweeps(wf_solver* h, int n, bool allow_fast) {
             wf::launch_pres_sweep(P, h->st, h->fl, src, h->Dv, h->Dp, h->bp, h->pcb[h->iPC]);
         WF_CHECK_LAUNCH();
         h->pc_zero = false;
-        if (resid && k % h->cfg.pres_res_interval == 0) {
-            wf::launch_pres_residual(P, h->st, h->Dp, h->pcb[h->iPC], src, h->part, h->dsum);
-            double s = 0.0;
-            WF_TRY(read_residual(h, &s));
-            h->res_pres = (float)std::sqrt(s / double(P.N));
-            if (h->res_pres < h->cfg.pres_tol) break;
-        }
+        bool done = false;
+        if (resid && k % h->cfg.pres_res_interval == 0) WF_TRY(pres_converged(h, h->pcb[h->iPC], src, &done));
+        if (done) break;
+        std::swap(h->iPCL, h->iPC);
+        if (!chip) continue;
+        const int interval = h->cfg.pres_res_interval;
+        const int m = std::min((k / interval + 1) * interval, n - 1) - k;  // sweeps up to the next check
+        if (m < 2 || !wf::pres_sweeps_on_chip(h, m, coef_done, true)) continue;
+        coef_done = true;
+        k += m;
+        if (k % interval == 0) WF_TRY(pres_converged(h, h->pcb[h->iPC], h->pcb[h->iPCL], &done));
+        if (done) break;
         std::swap(h->iPCL, h->iPC);
     }
     std::swap(h->iPCL, h->iPC);

@@ -109,6 +109,12 @@ __host__ __device__ constexpr int plane_of(int R) {
 __host__ __device__ constexpr int rim_of(const ResPlan& p) { return 2 * (p.bx + p.by) - 4; }
 __host__ __device__ constexpr int inner0_of(const ResPlan& p) { return (rim_of(p) + 4 + 31) / 32 * 32; }
 __host__ __device__ constexpr int inner_of(const ResPlan& p) { return (p.bx - 2) * (p.by - 2); }
+// Halo cells the busiest thread fetches: the rim + 4 halo cells of a plane go
+// to as many threads, NT / (rim + 4) planes at a time.
+__host__ __device__ constexpr int fetches_of(const ResPlan& p) {
+    const int G = NT / (rim_of(p) + 4);
+    return (p.bz + G - 1) / G;
+}
 __host__ __device__ constexpr int slots_of(const ResPlan& p) {
     return p.bz * rim_of(p) + 2 * (inner0_of(p) + inner_of(p));
 }
@@ -152,14 +158,22 @@ struct Links {
     int se;       // its cell on the rim
     int su, sd;   // its top and bottom cell
     int ru, rd;   // the cells above and below its column
-    int re, he;   // the halo cell it fetches: packet and shared offset
+    // the halo cells it fetches, of planes g, g + G, ...: packet and shared
+    // offset of the first (re -1: outside the domain), their steps, how many
+    int re, he, rstep, hstep, rn;
 };
-__device__ __forceinline__ Links make_links(const Box& b, const ResPlan& pl, bool own) {
+constexpr int kFetch = 4;  // halo cells a thread fetches at most in the momentum loop
+// `groups`: planes whose halo cells are fetched by different threads.
+__device__ __forceinline__ Links make_links(const Box& b, const ResPlan& pl, bool own, int groups) {
     Links l;
     const int tid = threadIdx.x, mine = b.id * b.slots;
     const int ix = b.id % pl.px, iy = (b.id / pl.px) % pl.py, iz = b.id / (pl.px * pl.py);
     l.se = l.su = l.sd = l.ru = l.rd = l.re = -1;
     l.he = 0;
+    const int G = groups, g = tid / (b.rim + 4), e = tid % (b.rim + 4);
+    l.rstep = G * b.rim;
+    l.hstep = G * plane_of(pl.bz);
+    l.rn = g < G && g < pl.bz ? (pl.bz - 1 - g) / G + 1 : 0;
     const int top = pl.bz * b.rim, layer = pl.px * pl.py, half = b.inner0 + inner_of(pl);
     if (own) {
         if (tid < b.rim && layer > 1) l.se = mine + tid;
@@ -172,31 +186,29 @@ __device__ __forceinline__ Links make_links(const Box& b, const ResPlan& pl, boo
             l.rd = (b.id - layer) * b.slots + top + tid;
         }
     }
-    // halo cell e = tid of the E, W, N, S side and the rim thread of the
-    // neighbour box that owns it
-    if (tid < b.rim + 4) {
-        const int bx = pl.bx, by = pl.by;
-        int from = -1, t = 0, hx = 0, hy = 0;
-        if (tid < by) {
-            if (ix + 1 < pl.px) from = b.id + 1;
-            hx = bx; hy = tid;
-            t = by + tid;
-        } else if (tid < 2 * by) {
-            if (ix > 0) from = b.id - 1;
-            hx = -1; hy = tid - by;
-            t = hy;
-        } else if (tid < 2 * by + bx) {
-            if (iy + 1 < pl.py) from = b.id + pl.px;
-            hx = tid - 2 * by; hy = by;
-            t = hx == bx - 1 ? 0 : hx == 0 ? by : 2 * by + bx - 2 + hx - 1;
-        } else {
-            if (iy > 0) from = b.id - pl.px;
-            hx = tid - 2 * by - bx; hy = -1;
-            t = hx == bx - 1 ? by - 1 : hx == 0 ? 2 * by - 1 : 2 * by + hx - 1;
-        }
-        l.he = (hy + 1) * b.sx + hx + 1;
-        if (from >= 0) l.re = from * b.slots + t;
+    // halo cell e of the E, W, N, S side and the rim thread of the neighbour
+    // box that owns it
+    const int bx = pl.bx, by = pl.by;
+    int from = -1, t = 0, hx = 0, hy = 0;
+    if (e < by) {
+        if (ix + 1 < pl.px) from = b.id + 1;
+        hx = bx; hy = e;
+        t = by + e;
+    } else if (e < 2 * by) {
+        if (ix > 0) from = b.id - 1;
+        hx = -1; hy = e - by;
+        t = hy;
+    } else if (e < 2 * by + bx) {
+        if (iy + 1 < pl.py) from = b.id + pl.px;
+        hx = e - 2 * by; hy = by;
+        t = hx == bx - 1 ? 0 : hx == 0 ? by : 2 * by + bx - 2 + hx - 1;
+    } else {
+        if (iy > 0) from = b.id - pl.px;
+        hx = e - 2 * by - bx; hy = -1;
+        t = hx == bx - 1 ? by - 1 : hx == 0 ? 2 * by - 1 : 2 * by + hx - 1;
     }
+    l.he = (hy + 1) * b.sx + hx + 1 + g * plane_of(pl.bz);
+    if (from >= 0 && l.rn > 0) l.re = from * b.slots + t + g * b.rim;
     return l;
 }
 
@@ -260,6 +272,12 @@ __device__ __forceinline__ void epoch_end(unsigned* ctl, unsigned base, unsigned
     }
 }
 
+// kPasses: the uniform grid with the rounding of the four-sweep passes (their
+// compiled sum fuses the first product, not the second, into the add);
+// kOrdered: with that of the one-sweep reference-form kernel; kStretched: six
+// coefficients a cell, rounded as kOrdered.
+enum class Form { kPasses, kOrdered, kStretched };
+
 struct PresArgs {
     int nx, ny, nz, n;
     ResPlan pl;
@@ -285,9 +303,10 @@ static_assert(pres_smem(8) <= kSmemMax && pres_smem(10) <= kSmemMax && pres_smem
 // what every sweep does (its code has to stay in the instruction cache: with
 // the last sweep's and the optional stores inside, a sweep of an 11 x 8 x 8 box
 // alone took 1980 cycles instead of 300); the last sweep follows it.
-template <int R, bool NU, bool STACK>
+template <int R, Form F, bool STACK>
 __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ PresArgs a) {
     extern __shared__ __align__(16) float sm[];
+    constexpr bool NU = F == Form::kStretched;
     constexpr bool kShared = R > kRegR;
     constexpr int PS = plane_of(R);
     const unsigned base = epoch_begin(a.ctl);
@@ -302,7 +321,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
     const bool inxy = own && x < a.nx && y < a.ny;
     const int i0 = inxy ? (b.z0 * a.ny + y) * a.nx + x : 0;
     const int o0 = (ly + 1) * b.sx + lx + 1;
-    const Links l = make_links(b, a.pl, own);
+    const Links l = make_links(b, a.pl, own, 1);
     // the input iterate with its halo, zero outside the domain
     for (int o = tid; o < 2 * R * PS; o += NT) sm[o] = 0.f;
     __syncthreads();
@@ -317,7 +336,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
         }
         if (inxy && b.z0 > 0) hd = __ldg(a.pin + i0 - sxy);
         if (inxy && b.z0 + R < a.nz) hu = __ldg(a.pin + i0 + R * sxy);
-        if (tid < b.rim + 4) {
+        if (tid < b.rim + 4) {  // the threads that fetch from plane 0 on
             const int hy = b.y0 + l.he / b.sx - 1, hx = b.x0 + l.he % b.sx - 1;
             if (hx >= 0 && hx < a.nx && hy >= 0 && hy < a.ny)
                 for (int r = 0; r < R && b.z0 + r < a.nz; ++r)
@@ -360,9 +379,8 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
     auto inv_of = [&](int r) { return kShared ? sai[r * NT + tid] : ai[kShared ? 0 : r]; };
     auto cell = [&](const float* q, int r, float up, float below) {
         const float *qn = q + b.sx, *qs = q - b.sx;
-        // the first two products in the rounding of the pass kernel of each grid
         float acc;
-        if (NU) {
+        if (F != Form::kPasses) {
             acc = __fmaf_rn(-cW[r], q[r * PS - 1], __fmul_rn(-cE[r], q[r * PS + 1]));
         } else {
             acc = -(cE[r] * q[r * PS + 1]);
@@ -475,47 +493,32 @@ struct VelArgs {
     int* status;
 };
 
-// receive() for three components.
-template <int R, bool RIM>
-__device__ __forceinline__ bool receive3(const Links& l, int rim, float* v, const Packet3* pk, unsigned ep, float hu[3],
+// receive() for three components, CS floats apart in the shared box.  Every
+// thread takes a share of the x / y halo, so that one trip fetches it (a rim
+// thread's R packets of four words do not fit beside the coefficients: 1.58 ->
+// 1.38 us a sweep on 64 x 32 x 48, 3.72 -> 3.38 on 100 x 50 x 100; the pressure
+// loop, whose rim threads hold theirs, lost 5 % by it).  nf: fetches of the
+// busiest thread.
+template <int CS>
+__device__ __forceinline__ bool receive3(const Links& l, int nf, float* v, const Packet3* pk, unsigned ep, float hu[3],
                                          float hd[3]) {
-    const bool nu = l.ru >= 0, nd = l.rd >= 0, ne = RIM && l.re >= 0;
+    const bool nu = l.ru >= 0, nd = l.rd >= 0, ne = l.re >= 0;
     const Packet3 *pu = pk + (nu ? l.ru : 0), *pd = pk + (nd ? l.rd : 0), *pe = pk + (ne ? l.re : 0);
-    constexpr int PS = plane_of(R);
+    Packet3 w[kFetch], wu, wd;
     int left = kRounds;
     bool ok;
-    if (RIM) {
-        // the edge cells first: they arrive last
-        constexpr int U = R <= 4 ? R : (R + 1) / 2;
-#pragma unroll
-        for (int r0 = 0; r0 < R; r0 += U) {
-            Packet3 w[U];
-            do {
-#pragma unroll
-                for (int q = 0; q < U; ++q) w[q] = get3(pe + (r0 + q < R ? r0 + q : R - 1) * rim);
-                ok = true;
-#pragma unroll
-                for (int q = 0; q < U; ++q) ok = ok && (unsigned)(w[q].hi >> 32) == ep;
-                ok = ok || !ne;
-            } while (!__all_sync(0xffffffffu, ok) && --left);
-            if (left == 0) return false;
-            if (ne) {
-#pragma unroll
-                for (int q = 0; q < U; ++q)
-                    if (r0 + q < R) {
-                        float* o = v + l.he + (r0 + q) * PS;
-                        o[0] = __uint_as_float((unsigned)w[q].lo);
-                        o[R * PS] = __uint_as_float((unsigned)(w[q].lo >> 32));
-                        o[2 * R * PS] = __uint_as_float((unsigned)w[q].hi);
-                    }
-            }
-        }
-    }
-    Packet3 wu, wd;
     do {
         wu = get3(pu);
         wd = get3(pd);
+#pragma unroll
+        for (int q = 0; q < kFetch; ++q)
+            if (q < nf) w[q] = get3(pe + (q < l.rn ? q : 0) * l.rstep);
         ok = (!nu || (unsigned)(wu.hi >> 32) == ep) && (!nd || (unsigned)(wd.hi >> 32) == ep);
+        bool oke = true;
+#pragma unroll
+        for (int q = 0; q < kFetch; ++q)
+            if (q < nf) oke = oke && (unsigned)(w[q].hi >> 32) == ep;
+        ok = ok && (oke || !ne);
     } while (!__all_sync(0xffffffffu, ok) && --left);
     if (left == 0) return false;
     hu[0] = nu ? __uint_as_float((unsigned)wu.lo) : 0.f;
@@ -524,6 +527,16 @@ __device__ __forceinline__ bool receive3(const Links& l, int rim, float* v, cons
     hd[0] = nd ? __uint_as_float((unsigned)wd.lo) : 0.f;
     hd[1] = nd ? __uint_as_float((unsigned)(wd.lo >> 32)) : 0.f;
     hd[2] = nd ? __uint_as_float((unsigned)wd.hi) : 0.f;
+    if (ne) {
+#pragma unroll
+        for (int q = 0; q < kFetch; ++q)
+            if (q < nf && q < l.rn) {
+                float* o = v + l.he + q * l.hstep;
+                o[0] = __uint_as_float((unsigned)w[q].lo);
+                o[CS] = __uint_as_float((unsigned)(w[q].lo >> 32));
+                o[2 * CS] = __uint_as_float((unsigned)w[q].hi);
+            }
+    }
     return true;
 }
 
@@ -539,12 +552,12 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
     const int sxy = a.nx * a.ny;
     const size_t N = (size_t)sxy * a.nz;
     int lx, ly;
-    const bool own = column_of(b, a.pl, tid, lx, ly), rim = tid < b.inner0;
+    const bool own = column_of(b, a.pl, tid, lx, ly);
     const int x = b.x0 + lx, y = b.y0 + ly;
     const bool inxy = own && x < a.nx && y < a.ny;
     const int i0 = inxy ? (b.z0 * a.ny + y) * a.nx + x : 0;
     const int o0 = (ly + 1) * b.sx + lx + 1;
-    const Links l = make_links(b, a.pl, own);
+    const Links l = make_links(b, a.pl, own, NT / (b.rim + 4));
     // the input iterate with its halo, zero outside the domain
     for (int o = tid; o < 3 * CS; o += NT) sm[o] = 0.f;
     __syncthreads();
@@ -639,7 +652,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
     Packet3 *pk = a.pk, *pk_next = a.pk + a.half;
     unsigned ep = base;
     bool bad = false;
-    const bool has_halo = gridDim.x > 1 && (tid & ~31) < b.inner0 + inner_of(a.pl);
+    const int nf = fetches_of(a.pl);
     for (int k = 1; k < a.n; ++k) {
         ++ep;
         ends();
@@ -658,8 +671,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
 #pragma unroll
                 for (int r = 0; r < R; ++r) cur[c * CS + r * PS] = u[c][r];
         }
-        if (has_halo)
-            bad = rim ? !receive3<R, true>(l, b.rim, sm, pk, ep, hu, hd) : !receive3<R, false>(l, b.rim, sm, pk, ep, hu, hd);
+        if (gridDim.x > 1) bad = !receive3<CS>(l, nf, sm, pk, ep, hu, hd);
         if (__syncthreads_or(bad)) break;
         Packet3* t = pk;
         pk = pk_next;
@@ -683,22 +695,22 @@ constexpr int kNuPresR[] = {2, 3, 4, 6, 8};
 constexpr int kVelR[] = {2, 3, 4, 6, 8};
 
 using PresKernel = void (*)(const PresArgs);
-template <bool NU, bool STACK>
+template <Form F, bool STACK>
 PresKernel pres_kernel(int R) {
     switch (R) {
-        case 2: return k_res_pres<2, NU, STACK>;
-        case 3: return k_res_pres<3, NU, STACK>;
-        case 4: return k_res_pres<4, NU, STACK>;
-        case 6: return k_res_pres<6, NU, STACK>;
-        case 8: return k_res_pres<8, NU, STACK>;
+        case 2: return k_res_pres<2, F, STACK>;
+        case 3: return k_res_pres<3, F, STACK>;
+        case 4: return k_res_pres<4, F, STACK>;
+        case 6: return k_res_pres<6, F, STACK>;
+        case 8: return k_res_pres<8, F, STACK>;
         default: break;
     }
-    if constexpr (!NU) {
+    if constexpr (F != Form::kStretched) {
         switch (R) {
-            case 10: return k_res_pres<10, NU, STACK>;
-            case 12: return k_res_pres<12, NU, STACK>;
-            case 14: return k_res_pres<14, NU, STACK>;
-            case 16: return k_res_pres<16, NU, STACK>;
+            case 10: return k_res_pres<10, F, STACK>;
+            case 12: return k_res_pres<12, F, STACK>;
+            case 14: return k_res_pres<14, F, STACK>;
+            case 16: return k_res_pres<16, F, STACK>;
             default: break;
         }
     }
@@ -738,7 +750,8 @@ ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M]) {
                 ResPlan pl;
                 pl.bx = bx; pl.by = by; pl.bz = R;
                 pl.px = px; pl.py = py; pl.pz = pz;
-                if (inner0_of(pl) + inner_of(pl) > NT || (bx + kPad) * (by + 2) > plane_of(R)) continue;
+                if (inner0_of(pl) + inner_of(pl) > NT || (bx + kPad) * (by + 2) > plane_of(R) || fetches_of(pl) > kFetch)
+                    continue;
                 const double halo = 2.0 * ((px > 1 ? by * R : 0) + (py > 1 ? bx * R : 0) + (pz > 1 ? bx * by : 0));
                 const double c = R * (60.0 + 0.6 * (inner0_of(pl) / 32 + (inner_of(pl) + 31) / 32)) + 0.03 * halo;
                 if (c < cost) {
@@ -777,10 +790,11 @@ int resident_setup(const Resident& r) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
     };
     if (r.pres.bz > 0) {
-        opt_in(pres_kernel<false, false>(r.pres.bz));
-        opt_in(pres_kernel<false, true>(r.pres.bz));
+        opt_in(pres_kernel<Form::kPasses, false>(r.pres.bz));
+        opt_in(pres_kernel<Form::kPasses, true>(r.pres.bz));
+        opt_in(pres_kernel<Form::kOrdered, false>(r.pres.bz));
     }
-    if (r.nupres.bz > 0) opt_in(pres_kernel<true, false>(r.nupres.bz));
+    if (r.nupres.bz > 0) opt_in(pres_kernel<Form::kStretched, false>(r.nupres.bz));
     if (r.vel.bz > 0) opt_in(vel_kernel(r.vel.bz));
     return e == cudaSuccess ? WF_OK : WF_ERR_CUDA;
 }
@@ -819,10 +833,9 @@ void resident_free(Resident* r) {
 }
 
 namespace {
-template <bool NU>
-cudaError_t launch_pres(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w, const float* c,
-                        const float* ainv, const float* rhs, const float* pin, float* pout, float* pprev,
-                        float* stack, int n, int* status) {
+cudaError_t launch_pres(PresKernel k, const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w,
+                        const float* c, const float* ainv, const float* rhs, const float* pin, float* pout,
+                        float* pprev, float* stack, int n, int* status) {
     PresArgs a = {};
     a.nx = P.nx; a.ny = P.ny; a.nz = P.nz; a.n = n;
     a.pl = pl;
@@ -832,7 +845,6 @@ cudaError_t launch_pres(const Params& P, cudaStream_t st, const ResPlan& pl, con
     a.half = packets(pl);
     a.ctl = w.ctl;
     a.status = status;
-    const PresKernel k = !NU && stack ? pres_kernel<false, true>(pl.bz) : pres_kernel<NU, false>(pl.bz);
     const cudaError_t e = launch_coop((const void*)k, pl.boxes(), pres_smem(pl.bz), st, &a);
     if (e == cudaSuccess) WF_COUNT_LAUNCH();
     else cudaGetLastError();
@@ -842,14 +854,18 @@ cudaError_t launch_pres(const Params& P, cudaStream_t st, const ResPlan& pl, con
 
 cudaError_t launch_res_pres(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w, const float* c3,
                             const float* ainv, const float* rhs, const float* pin, float* pout, float* pprev,
-                            float* stack, int n, int* status) {
-    return launch_pres<false>(P, st, pl, w, c3, ainv, rhs, pin, pout, pprev, stack, n, status);
+                            float* stack, int n, int* status, bool ordered) {
+    const PresKernel k = stack     ? pres_kernel<Form::kPasses, true>(pl.bz)
+                         : ordered ? pres_kernel<Form::kOrdered, false>(pl.bz)
+                                   : pres_kernel<Form::kPasses, false>(pl.bz);
+    return launch_pres(k, P, st, pl, w, c3, ainv, rhs, pin, pout, pprev, stack, n, status);
 }
 
 cudaError_t launch_res_nupres(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w,
                               const float* coef, const float* bp, const float* pin, float* pout, float* pprev, int n,
                               int* status) {
-    return launch_pres<true>(P, st, pl, w, coef, coef + 6 * (size_t)P.N, bp, pin, pout, pprev, nullptr, n, status);
+    return launch_pres(pres_kernel<Form::kStretched, false>(pl.bz), P, st, pl, w, coef, coef + 6 * (size_t)P.N, bp, pin,
+                       pout, pprev, nullptr, n, status);
 }
 
 cudaError_t launch_res_vel(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w, const float* A,

@@ -46,11 +46,12 @@ void resident_free(Resident* r);
 // equations in one cooperative launch, from pin (nullptr: zero), with the
 // iterates of k_pres_msweep / k_pres_tma4 bit for bit.  pout receives iterate
 // n on fluid cells, pprev (nullable) iterate n - 1; stack (nullable) every
-// iterate k = 1..n of every cell at stack + k N.  rhs nullptr: 0.  A bounded
-// wait that runs out sets *status to 1.
+// iterate k = 1..n of every cell at stack + k N.  rhs nullptr: 0.  ordered
+// (without a stack): the iterates of the one-sweep kernel launch_pres_sweep
+// instead.  A bounded wait that runs out sets *status to 1.
 cudaError_t launch_res_pres(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w, const float* c3,
                             const float* ainv, const float* rhs, const float* pin, float* pout, float* pprev,
-                            float* stack, int n, int* status);
+                            float* stack, int n, int* status, bool ordered = false);
 // The same for the non-uniform grid: six face coefficients and 1/Dp
 // (coef, kNuCoefPlanes planes), right-hand side bp; the iterates of
 // k_nu_pres_sweep bit for bit.

@@ -1075,22 +1075,41 @@ int record_pres_loop(wf_solver* h, int n, const float* rhs) {
 
 }  // namespace
 
+namespace {
+// The whole loop on chip: output and iterate n - 1 go to the two buffers
+// that are not the input.
+template <typename Launch>
+bool pres_loop(wf_solver* h, bool keep_prev, Launch launch) {
+    const int in = h->pc_zero ? -1 : h->iPCL, out = in == 0 ? 1 : 0, prev = in < 0 ? 1 : 3 - in - out;
+    if (launch(in < 0 ? nullptr : h->pcb[in], h->pcb[out], keep_prev ? h->pcb[prev] : nullptr) != cudaSuccess)
+        return false;
+    h->pc_zero = false;
+    h->iPC = out;
+    h->iPCL = prev;
+    return true;
+}
+}  // namespace
+
+bool pres_sweeps_on_chip(wf_solver* h, int n, bool coef_done, bool keep_prev) {
+    const size_t N = h->P.N;
+    if (!h->nonuniform && !coef_done) pres_coef(h, /*piso=*/false);
+    return pres_loop(h, keep_prev, [&](const float* in, float* out, float* prev) {
+        return h->nonuniform ? launch_res_nupres(h->P, h->st, h->res.nupres, h->res.work, h->nucoef, h->bp, in, out,
+                                                 prev, n, h->dstat)
+                             : launch_res_pres(h->P, h->st, h->res.pres, h->res.work, h->pcoef, h->pcoef + 3 * N,
+                                               h->bp, in, out, prev, nullptr, n, h->dstat, /*ordered=*/true);
+    });
+}
+
 int pres_sweeps_fast(wf_solver* h, int n, bool piso) {
     const float* rhs = pres_coef(h, piso);
     if (h->rec) return record_pres_loop(h, n, rhs);
-    if (n >= 2 && loops_on_chip(h, h->res.pres)) {
-        // the whole loop on chip: output and iterate n - 1 go to the two
-        // buffers that are not the input
-        const int in = h->pc_zero ? -1 : h->iPCL, out = in == 0 ? 1 : 0, prev = in < 0 ? 1 : 3 - in - out;
-        if (launch_res_pres(h->P, h->st, h->res.pres, h->res.work, h->pcoef, h->pcoef + 3 * (size_t)h->P.N, rhs,
-                            in < 0 ? nullptr : h->pcb[in], h->pcb[out], h->in_step ? nullptr : h->pcb[prev], nullptr,
-                            n, h->dstat) == cudaSuccess) {
-            h->pc_zero = false;
-            h->iPC = out;
-            h->iPCL = prev;
-            return WF_OK;
-        }
-    }
+    if (n >= 2 && loops_on_chip(h, h->res.pres) &&
+        pres_loop(h, !h->in_step, [&](const float* in, float* out, float* prev) {
+            return launch_res_pres(h->P, h->st, h->res.pres, h->res.work, h->pcoef, h->pcoef + 3 * (size_t)h->P.N, rhs,
+                                   in, out, prev, nullptr, n, h->dstat);
+        }))
+        return WF_OK;
     const int kmax = std::min(std::max(h->pres_k, 1), 4);
     if (kmax == 1) {
         for (int k = 0; k < n; ++k) {

@@ -20,6 +20,13 @@ int vel_sweeps_fast(wf_solver* h, int n);
 // or CSPisoPresCorrection (piso = true, :1493-1514) with the same rotation.
 int pres_sweeps_fast(wf_solver* h, int n, bool piso);
 
+// n >= 2 sweeps of CSPresCorrectRhieChow on chip (loops_on_chip holds), with
+// the iterates of the one-sweep kernels launch_pres_sweep /
+// launch_nu_pres_sweep bit for bit; keep_prev: pcb[iPCL] then holds iterate
+// n - 1.  coef_done: the loop's 1/Dp is in place.  False where the launch
+// failed: nothing was run.
+bool pres_sweeps_on_chip(wf_solver* h, int n, bool coef_done, bool keep_prev);
+
 // Explicit-pointer launchers of the fast Jacobi building blocks: momentum
 // coefficients A (6 planes) and 1/D (3), one momentum sweep, pressure face
 // coefficients c_E/c_N/c_U, 1/Dp, PISO diagonal and right-hand side.  The
