@@ -734,8 +734,11 @@ VelKernel vel_kernel(int R) {
 // 1.45-1.67 with 8 in 4 to 8 warps, 1.75 in 16 warps, 2.3 with 12, 2.6-2.9 with
 // 14, 3.4 with 16: the cells of a thread weigh most (a warp works through
 // them one after another), then the warps, then the halo.
+// shared: beside other cases' loops the product of a sweep's time and the
+// multiprocessors it holds counts instead, so that as many loops as possible
+// run at once.
 template <size_t M>
-ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M]) {
+ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], bool shared = false) {
     ResPlan best;
     double cost = 1e30;
     sms = std::min(sms, kMaxBoxes);
@@ -753,7 +756,8 @@ ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M]) {
                 if (inner0_of(pl) + inner_of(pl) > NT || (bx + kPad) * (by + 2) > plane_of(R) || fetches_of(pl) > kFetch)
                     continue;
                 const double halo = 2.0 * ((px > 1 ? by * R : 0) + (py > 1 ? bx * R : 0) + (pz > 1 ? bx * by : 0));
-                const double c = R * (60.0 + 0.6 * (inner0_of(pl) / 32 + (inner_of(pl) + 31) / 32)) + 0.03 * halo;
+                double c = R * (60.0 + 0.6 * (inner0_of(pl) / 32 + (inner_of(pl) + 31) / 32)) + 0.03 * halo;
+                if (shared) c = (500.0 + c) * pl.boxes();
                 if (c < cost) {
                     cost = c;
                     best = pl;
@@ -795,7 +799,9 @@ int resident_setup(const Resident& r) {
         opt_in(pres_kernel<Form::kOrdered, false>(r.pres.bz));
     }
     if (r.nupres.bz > 0) opt_in(pres_kernel<Form::kStretched, false>(r.nupres.bz));
-    if (r.vel.bz > 0) opt_in(vel_kernel(r.vel.bz));
+    if (r.pres_shared.bz > 0) opt_in(pres_kernel<Form::kPasses, false>(r.pres_shared.bz));
+    for (const ResPlan& p : {r.vel, r.vel_shared})
+        if (p.bz > 0) opt_in(vel_kernel(p.bz));
     return e == cudaSuccess ? WF_OK : WF_ERR_CUDA;
 }
 
@@ -803,13 +809,16 @@ void resident_plan(const Params& P, int sms, Resident* r) {
     r->pres = make_plan(P, sms, kPresR);
     r->nupres = make_plan(P, sms, kNuPresR);
     r->vel = make_plan(P, sms, kVelR);
+    r->pres_shared = make_plan(P, sms, kPresR, true);
+    r->vel_shared = make_plan(P, sms, kVelR, true);
 }
 
 void resident_alloc(Resident* r, cudaStream_t st) {
     // both parities of the pressure packets, then of the momentum packets
     // (apart: a momentum packet's words must not be read as pressure
     // packets), then the epoch words
-    const size_t np = 2 * std::max(packets(r->pres), packets(r->nupres)), nv = 2 * packets(r->vel);
+    const size_t np = 2 * std::max({packets(r->pres), packets(r->nupres), packets(r->pres_shared)}),
+                 nv = 2 * std::max(packets(r->vel), packets(r->vel_shared));
     if (np + nv == 0 || r->work.pk) return;
     const size_t bytes = np * sizeof(unsigned long long) + nv * sizeof(Packet3) + 16;
     void* pk = nullptr;

@@ -28,6 +28,7 @@ struct Resident {
     ResPlan pres;      // uniform pressure loops
     ResPlan nupres;    // non-uniform pressure loop
     ResPlan vel;       // momentum loop
+    ResPlan pres_shared, vel_shared;  // the same beside other cases' loops: fewest multiprocessors
     ResWork work;
     bool ok(const ResPlan& p) const { return p.bz > 0 && work.pk != nullptr; }
 };

@@ -127,14 +127,22 @@ struct wf_solver {
 };
 
 namespace wf {
-// Cells from which a case of a batch runs its loops on chip.  Such a loop
-// takes the whole GPU, so the cases' loops run one after another; passes of
-// small cases fill the GPU together.  Measured per batched step: 16 cases of
-// 0.06-0.21 M cells 3.37 ms in passes, 3.77 ms on chip; 16 cases of 0.7-1.75 M
-// cells 20.6 ms in passes, 19.4 ms with the ones that fit on chip.
-constexpr int kBatchOnChipCells = 500000;
-inline bool loops_on_chip(const wf_solver* h, const ResPlan& p) {
-    return h->resident && h->dstat && h->res.ok(p) && (!h->in_batch || h->P.N >= kBatchOnChipCells);
+inline bool loops_on_chip(const wf_solver* h, const ResPlan& p) { return h->resident && h->dstat && h->res.ok(p); }
+// The loops' splits: the fastest alone; beside the other cases of a batch the
+// one that holds the fewest multiprocessors for its time, where it leaves at
+// least half of them to the others.  A larger case keeps its pressure split for
+// a lone case and its momentum passes.  Us a batched step: 16 cases of 0.06-0.21 M
+// cells 3370 in passes, 3770 with lone splits (one loop after another), 2061
+// with shared ones; 16 cases of 0.7-1.75 M cells 20600 in passes, 19600 with this
+// rule, 28800 with shared splits whatever their size (loops of more than half
+// the GPU each wait for it to empty).
+inline const ResPlan& pres_plan(const wf_solver* h) {
+    return h->in_batch && 2 * h->res.pres_shared.boxes() <= h->num_sms ? h->res.pres_shared : h->res.pres;
+}
+inline const ResPlan& vel_plan(const wf_solver* h) {
+    static const ResPlan none;
+    if (!h->in_batch) return h->res.vel;
+    return 2 * h->res.vel_shared.boxes() <= h->num_sms ? h->res.vel_shared : none;
 }
 
 // Step-graph plumbing shared by the single-handle and the batched step.

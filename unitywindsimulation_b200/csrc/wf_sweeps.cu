@@ -926,7 +926,7 @@ int record_vel_loop(wf_solver* h, int n) {
 int vel_sweeps_fast(wf_solver* h, int n) {
     vel_coef(h);
     if (h->rec) return record_vel_loop(h, n);
-    if (n >= 2 && loops_on_chip(h, h->res.vel)) {
+    if (n >= 2 && loops_on_chip(h, vel_plan(h))) {
         // the whole loop on chip, into two buffers that are neither its input
         // nor velFieldLastTime
         const size_t N = h->P.N;
@@ -934,7 +934,7 @@ int vel_sweeps_fast(wf_solver* h, int n) {
         int out = 0, prev = 0;
         while (out == h->iT || out == in) ++out;
         while (prev == h->iT || prev == in || prev == out) ++prev;
-        if (launch_res_vel(h->P, h->st, h->res.vel, h->res.work, h->vcoef, h->vcoef + 6 * N, h->bv, h->vb[in],
+        if (launch_res_vel(h->P, h->st, vel_plan(h), h->res.work, h->vcoef, h->vcoef + 6 * N, h->bv, h->vb[in],
                            h->vb[out], h->in_step ? nullptr : h->vb[prev], n, h->dstat) == cudaSuccess) {
             h->iF = out;
             h->iI = prev;
@@ -1104,9 +1104,9 @@ bool pres_sweeps_on_chip(wf_solver* h, int n, bool coef_done, bool keep_prev) {
 int pres_sweeps_fast(wf_solver* h, int n, bool piso) {
     const float* rhs = pres_coef(h, piso);
     if (h->rec) return record_pres_loop(h, n, rhs);
-    if (n >= 2 && loops_on_chip(h, h->res.pres) &&
+    if (n >= 2 && loops_on_chip(h, pres_plan(h)) &&
         pres_loop(h, !h->in_step, [&](const float* in, float* out, float* prev) {
-            return launch_res_pres(h->P, h->st, h->res.pres, h->res.work, h->pcoef, h->pcoef + 3 * (size_t)h->P.N, rhs,
+            return launch_res_pres(h->P, h->st, pres_plan(h), h->res.work, h->pcoef, h->pcoef + 3 * (size_t)h->P.N, rhs,
                                    in, out, prev, nullptr, n, h->dstat);
         }))
         return WF_OK;
@@ -1187,8 +1187,8 @@ int time_kernel(wf_solver* h, int which, int reps, bool flush, float* ms, double
     cudaEventCreate(&e1);
     float total = 0.f;
     // where the pressure loops run on chip one launch is a whole loop
-    const bool res_p = which == WF_KERNEL_PRES_SWEEP && loops_on_chip(h, h->res.pres) && h->cfg.pres_iters >= 2;
-    const bool res_v = which == WF_KERNEL_VEL_SWEEP && loops_on_chip(h, h->res.vel) && h->cfg.vel_iters >= 2;
+    const bool res_p = which == WF_KERNEL_PRES_SWEEP && loops_on_chip(h, pres_plan(h)) && h->cfg.pres_iters >= 2;
+    const bool res_v = which == WF_KERNEL_VEL_SWEEP && loops_on_chip(h, vel_plan(h)) && h->cfg.vel_iters >= 2;
     const int kv = res_v ? h->cfg.vel_iters : std::min(std::max(h->vel_k, 1), 2);
     const int kp = res_p ? h->cfg.pres_iters : std::min(std::max(h->pres_k, 1), 4);
     for (int r = 0; r < reps; ++r) {
@@ -1196,13 +1196,13 @@ int time_kernel(wf_solver* h, int which, int reps, bool flush, float* ms, double
         cudaEventRecord(e0, h->st);
         if (which == WF_KERNEL_VEL_SWEEP) {
             if (res_v)
-                launch_res_vel(P, h->st, h->res.vel, h->res.work, h->vcoef, h->vcoef + 6 * N, h->bv, a, b, nullptr, kv,
+                launch_res_vel(P, h->st, vel_plan(h), h->res.work, h->vcoef, h->vcoef + 6 * N, h->bv, a, b, nullptr, kv,
                                h->dstat);
             else if (kv > 1) launch_vmsweep(h, kv, a, b, nullptr);
             else launch_vel_sweep_fast(h, a, b);
         } else {
             if (res_p)
-                launch_res_pres(P, h->st, h->res.pres, h->res.work, h->pcoef, h->pcoef + 3 * N, rhs, a, b, nullptr,
+                launch_res_pres(P, h->st, pres_plan(h), h->res.work, h->pcoef, h->pcoef + 3 * N, rhs, a, b, nullptr,
                                 nullptr, kp, h->dstat);
             else if (kp > 1) launch_msweep(h, kp, rhs, a, b, nullptr);
             else launch_pres_sweep_fast(h, rhs, a, b);
