@@ -162,7 +162,8 @@ struct Links {
     // offset of the first (re -1: outside the domain), their steps, how many
     int re, he, rstep, hstep, rn;
 };
-constexpr int kFetch = 4;  // halo cells a thread fetches at most in the momentum loop
+// Halo cells a thread fetches at most in the momentum loop of R cells a thread.
+__host__ __device__ constexpr int fetch_max(int R) { return R <= 4 ? 1 : 2; }
 // `groups`: planes whose halo cells are fetched by different threads.
 __device__ __forceinline__ Links make_links(const Box& b, const ResPlan& pl, bool own, int groups) {
     Links l;
@@ -495,30 +496,29 @@ struct VelArgs {
 
 // receive() for three components, CS floats apart in the shared box.  Every
 // thread takes a share of the x / y halo, so that one trip fetches it (a rim
-// thread's R packets of four words do not fit beside the coefficients: 1.58 ->
-// 1.38 us a sweep on 64 x 32 x 48, 3.72 -> 3.38 on 100 x 50 x 100; the pressure
-// loop, whose rim threads hold theirs, lost 5 % by it).  nf: fetches of the
-// busiest thread.
-template <int CS>
-__device__ __forceinline__ bool receive3(const Links& l, int nf, float* v, const Packet3* pk, unsigned ep, float hu[3],
+// thread's R packets of four words do not fit beside the coefficients; the
+// pressure loop, whose rim threads hold theirs, lost 5 % by it).  The share is
+// one packet up to R = 4 and two above, fixed at compile time: shares of up to
+// four behind a runtime count cost registers and a branch each.  us a sweep, rim
+// threads alone / up to four / now: 64 x 32 x 48 1.58 / 1.38 / 1.30, 72 x 40 x 72
+// - / 1.61 / 1.55, 100 x 50 x 100 3.72 / 3.38 / 2.96.
+template <int R>
+__device__ __forceinline__ bool receive3(const Links& l, float* v, const Packet3* pk, unsigned ep, float hu[3],
                                          float hd[3]) {
+    constexpr int F = fetch_max(R), CS = R * plane_of(R);
     const bool nu = l.ru >= 0, nd = l.rd >= 0, ne = l.re >= 0;
     const Packet3 *pu = pk + (nu ? l.ru : 0), *pd = pk + (nd ? l.rd : 0), *pe = pk + (ne ? l.re : 0);
-    Packet3 w[kFetch], wu, wd;
+    const int second = F > 1 && l.rn > 1 ? l.rstep : 0;
+    Packet3 w[F], wu, wd;
     int left = kRounds;
     bool ok;
     do {
         wu = get3(pu);
         wd = get3(pd);
-#pragma unroll
-        for (int q = 0; q < kFetch; ++q)
-            if (q < nf) w[q] = get3(pe + (q < l.rn ? q : 0) * l.rstep);
+        w[0] = get3(pe);
+        if (F > 1) w[F - 1] = get3(pe + second);
         ok = (!nu || (unsigned)(wu.hi >> 32) == ep) && (!nd || (unsigned)(wd.hi >> 32) == ep);
-        bool oke = true;
-#pragma unroll
-        for (int q = 0; q < kFetch; ++q)
-            if (q < nf) oke = oke && (unsigned)(w[q].hi >> 32) == ep;
-        ok = ok && (oke || !ne);
+        ok = ok && (!ne || ((unsigned)(w[0].hi >> 32) == ep && (unsigned)(w[F - 1].hi >> 32) == ep));
     } while (!__all_sync(0xffffffffu, ok) && --left);
     if (left == 0) return false;
     hu[0] = nu ? __uint_as_float((unsigned)wu.lo) : 0.f;
@@ -528,14 +528,15 @@ __device__ __forceinline__ bool receive3(const Links& l, int nf, float* v, const
     hd[1] = nd ? __uint_as_float((unsigned)(wd.lo >> 32)) : 0.f;
     hd[2] = nd ? __uint_as_float((unsigned)wd.hi) : 0.f;
     if (ne) {
+        // a thread with one halo cell fetches and writes it twice
+        const int at[2] = {l.he, l.he + (second ? l.hstep : 0)};
 #pragma unroll
-        for (int q = 0; q < kFetch; ++q)
-            if (q < nf && q < l.rn) {
-                float* o = v + l.he + q * l.hstep;
-                o[0] = __uint_as_float((unsigned)w[q].lo);
-                o[CS] = __uint_as_float((unsigned)(w[q].lo >> 32));
-                o[2 * CS] = __uint_as_float((unsigned)w[q].hi);
-            }
+        for (int q = 0; q < F; ++q) {
+            float* o = v + at[q];
+            o[0] = __uint_as_float((unsigned)w[q].lo);
+            o[CS] = __uint_as_float((unsigned)(w[q].lo >> 32));
+            o[2 * CS] = __uint_as_float((unsigned)w[q].hi);
+        }
     }
     return true;
 }
@@ -652,7 +653,6 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
     Packet3 *pk = a.pk, *pk_next = a.pk + a.half;
     unsigned ep = base;
     bool bad = false;
-    const int nf = fetches_of(a.pl);
     for (int k = 1; k < a.n; ++k) {
         ++ep;
         ends();
@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
 #pragma unroll
                 for (int r = 0; r < R; ++r) cur[c * CS + r * PS] = u[c][r];
         }
-        if (gridDim.x > 1) bad = !receive3<CS>(l, nf, sm, pk, ep, hu, hd);
+        if (gridDim.x > 1) bad = !receive3<R>(l, sm, pk, ep, hu, hd);
         if (__syncthreads_or(bad)) break;
         Packet3* t = pk;
         pk = pk_next;
@@ -738,7 +738,7 @@ VelKernel vel_kernel(int R) {
 // multiprocessors it holds counts instead, so that as many loops as possible
 // run at once.
 template <size_t M>
-ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], bool shared = false) {
+ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], bool momentum = false, bool shared = false) {
     ResPlan best;
     double cost = 1e30;
     sms = std::min(sms, kMaxBoxes);
@@ -753,7 +753,8 @@ ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], bool shared = fa
                 ResPlan pl;
                 pl.bx = bx; pl.by = by; pl.bz = R;
                 pl.px = px; pl.py = py; pl.pz = pz;
-                if (inner0_of(pl) + inner_of(pl) > NT || (bx + kPad) * (by + 2) > plane_of(R) || fetches_of(pl) > kFetch)
+                if (inner0_of(pl) + inner_of(pl) > NT || (bx + kPad) * (by + 2) > plane_of(R) ||
+                    rim_of(pl) + 4 > NT || (momentum && fetches_of(pl) > fetch_max(R)))
                     continue;
                 const double halo = 2.0 * ((px > 1 ? by * R : 0) + (py > 1 ? bx * R : 0) + (pz > 1 ? bx * by : 0));
                 double c = R * (60.0 + 0.6 * (inner0_of(pl) / 32 + (inner_of(pl) + 31) / 32)) + 0.03 * halo;
@@ -808,9 +809,9 @@ int resident_setup(const Resident& r) {
 void resident_plan(const Params& P, int sms, Resident* r) {
     r->pres = make_plan(P, sms, kPresR);
     r->nupres = make_plan(P, sms, kNuPresR);
-    r->vel = make_plan(P, sms, kVelR);
-    r->pres_shared = make_plan(P, sms, kPresR, true);
-    r->vel_shared = make_plan(P, sms, kVelR, true);
+    r->vel = make_plan(P, sms, kVelR, true);
+    r->pres_shared = make_plan(P, sms, kPresR, false, true);
+    r->vel_shared = make_plan(P, sms, kVelR, true, true);
 }
 
 void resident_alloc(Resident* r, cudaStream_t st) {
