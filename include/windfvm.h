@@ -485,7 +485,8 @@ int wf_get_blocking(const wf_solver* h, int* pres_k, int* vel_k);
 /* Tile shapes of the Jacobi kernels: rows of the pressure multi-sweep tile
  * (32: 32 x 32 tiles, one block per SM; 16: 32 x 16 tiles, two blocks per
  * SM, more tiles for small grids) and the block of the four-cell momentum
- * sweep (vel_bx * vel_by * vel_bz == 256 threads; default 32 x 4 x 2).
+ * sweep (vel_bx * vel_by * vel_bz == 256 threads; default: the one of 32 x 4 x 2,
+ * 16 x 8 x 2, 16 x 4 x 4 and 8 x 8 x 4 that leaves the fewest threads idle).
  * Results do not depend on them.  Drops the handle's captured step graphs.
  * No counterpart in the reference (its kernels are [numthreads(8,8,8)]). */
 int wf_set_tiles(wf_solver* h, int pres_rows, int vel_bx, int vel_by, int vel_bz);

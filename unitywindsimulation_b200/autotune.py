@@ -24,7 +24,7 @@ DEFAULT_CACHE = os.path.join(os.path.expanduser("~"), ".cache", "windfvm", "auto
 PRES_DEPTHS = (1, 2, 3, 4)
 PRES_ROWS = (32, 16)
 VEL_DEPTHS = (1, 2)
-VEL_BLOCKS = ((32, 4, 2), (32, 8, 1), (16, 8, 2), (64, 2, 2))
+VEL_BLOCKS = ((32, 4, 2), (32, 8, 1), (16, 8, 2), (64, 2, 2), (8, 8, 4))
 
 
 def _key(solver, device_name: str) -> str:

@@ -850,11 +850,6 @@ __global__ void k_objective(const __grid_constant__ Params P, const uint8_t* __r
     }
 }
 
-dim3 cblk() { return dim3(32, 4, 2); }
-dim3 cgrd(const Params& P) {
-    dim3 b = cblk();
-    return dim3((P.nx + b.x - 1) / b.x, (P.ny + b.y - 1) / b.y, (P.nz + b.z - 1) / b.z);
-}
 int lin_blocks(long long n) { return (int)((n + 255) / 256); }
 
 }  // namespace
@@ -1042,7 +1037,7 @@ int record_step(wf_adjoint* a, Tape& t, const float* u_in, const float* p_in, in
 void reverse_pres_loop(wf_adjoint* a, const float* ai, const float* c3, const float* sstack) {
     const Params& P = a->h->P;
     cudaStream_t st = a->st;
-    const dim3 g = wf::cgrd(P), bk = wf::cblk();
+    const dim3 g = wf::cells_grid(P), bk = wf::cells_block(P);
     const int n = a->nP;
     if (n == 0) {
         cudaMemsetAsync(a->rb, 0, a->N * sizeof(float), st);
@@ -1054,7 +1049,7 @@ void reverse_pres_loop(wf_adjoint* a, const float* ai, const float* c3, const fl
     if (n > 1) wf::launch_pres_stack(P, st, a->h->num_sms, c3, ai, nullptr, a->Wp, n - 1, false, tma_status(a->h),
                                      adj_resident(a));
     if (wf::quad_ok(P, {ai, a->Wp, sstack, a->rb, a->dgb, a->c3b})) {
-        const dim3 b4 = wf::cblk(), g4q((P.nx / 4 + b4.x - 1) / b4.x, (P.ny + b4.y - 1) / b4.y, (P.nz + b4.z - 1) / b4.z);
+        const dim3 b4 = wf::groups_block(P), g4q = wf::grid_for(P.nx / 4, P.ny, P.nz, b4);
         wf::k_adj_pacc4<<<g4q, b4, 0, st>>>(P, n, ai, a->Wp, sstack, a->rb, a->dgb, a->c3b);
     } else {
         wf::k_adj_pacc<<<g, bk, 0, st>>>(P, n, ai, a->Wp, sstack, a->rb, a->dgb, a->c3b);
@@ -1070,7 +1065,7 @@ int adjoint_step(wf_adjoint* a, const Tape& t, int phases) {
     cudaStream_t st = a->st;
     const size_t N = a->N;
     const size_t v = 3 * N * sizeof(float), s = N * sizeof(float);
-    const dim3 g = wf::cgrd(P), bk = wf::cblk();
+    const dim3 g = wf::cells_grid(P), bk = wf::cells_block(P);
     const wf::BndBar G = bnd_bar(a);
     WFA_CUDA(cudaMemsetAsync(a->uTb, 0, v, st));
     WFA_CUDA(cudaMemsetAsync(a->Db, 0, v, st));
@@ -1110,18 +1105,18 @@ int adjoint_step(wf_adjoint* a, const Tape& t, int phases) {
         wf::k_adj_vinit<<<wf::lin_blocks(3 * (long long)N), 256, 0, st>>>(3 * (long long)N, t.iD, a->ub,
                                                                            V(a, a->Wv, n));
         const bool v4 = n > 1 && wf::quad_ok(P, {a->AT, t.iD, V(a, a->Wv, n), V(a, a->Wv, n - 1)});
-        const dim3 g4((P.nx / 4 + bk.x - 1) / bk.x, (P.ny + bk.y - 1) / bk.y, (P.nz + bk.z - 1) / bk.z);
+        const dim3 b4 = wf::groups_block(P), g4 = wf::grid_for(P.nx / 4, P.ny, P.nz, b4);
         for (int k = n - 1; k >= 1; --k) {
             if (v4)
-                wf::k_adj_vsweepT4<<<g4, bk, 0, st>>>(P, a->AT, t.iD, V(a, a->Wv, k + 1), V(a, a->Wv, k));
+                wf::k_adj_vsweepT4<<<g4, b4, 0, st>>>(P, a->AT, t.iD, V(a, a->Wv, k + 1), V(a, a->Wv, k));
             else
                 wf::k_adj_vsweepT<false><<<g, bk, 0, st>>>(P, a->AT, t.iD, V(a, a->Wv, k + 1), nullptr,
                                                           V(a, a->Wv, k));
         }
         wf::k_adj_vsweepT<true><<<g, bk, 0, st>>>(P, a->AT, t.iD, V(a, a->Wv, 1), a->ub, a->uTb);
         if (wf::quad_ok(P, {a->Wv, t.uit, a->bb, a->Db, a->uTb})) {
-            const dim3 b4(32, 4, 1), g4q((P.nx / 4 + 31) / 32, (P.ny + 3) / 4, P.nz);
-            wf::k_adj_vacc4<<<g4q, b4, 0, st>>>(P, n, a->Wv, t.uit, a->bb, a->Db, a->uTb);
+            const dim3 bv(b4.x, 128 / b4.x, 1), gv = wf::grid_for(P.nx / 4, P.ny, P.nz, bv);
+            wf::k_adj_vacc4<<<gv, bv, 0, st>>>(P, n, a->Wv, t.uit, a->bb, a->Db, a->uTb);
         } else {
             wf::k_adj_vacc<<<g, bk, 0, st>>>(P, n, h->fl, a->Wv, t.uit, a->bb, a->Db, a->uTb);
         }

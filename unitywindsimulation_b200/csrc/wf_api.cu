@@ -716,6 +716,12 @@ int wf_create(const wf_config* cfg, int device, wf_solver** out) {
     P.les = cfg->turbulence == WF_TURB_SMAGORINSKY;
     P.compat = cfg->compat_flags;
     P.vec4 = h->vec4;
+    if (P.nx % 4 == 0) {
+        const dim3 b = wf::groups_block(P);
+        h->vel_blk[0] = (int)b.x;
+        h->vel_blk[1] = (int)b.y;
+        h->vel_blk[2] = (int)b.z;
+    }
 
     int s = WF_OK;
     auto fail = [&](int code) {

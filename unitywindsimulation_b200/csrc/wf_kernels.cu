@@ -1100,6 +1100,10 @@ int cell_grid_blocks(const Params& P) {
 }
 
 #define WF_LAUNCH(kernel, ...) \
+    (WF_COUNT_LAUNCH(), kernel<<<cells_grid(P), cells_block(P), 0, st>>>(P, __VA_ARGS__))
+// Kernels whose blocks leave partial sums: one shape whatever the grid, so
+// that the sums' order is fixed.
+#define WF_LAUNCH_SUMS(kernel, ...) \
     (WF_COUNT_LAUNCH(), kernel<<<cell_grid(P), cell_block(), 0, st>>>(P, __VA_ARGS__))
 
 void launch_wallfunc(const Params& P, cudaStream_t st, const uint8_t* fl, const float* uT, float* face) {
@@ -1169,19 +1173,19 @@ void launch_nbmask(const Params& P, cudaStream_t st, const uint8_t* fl, uint8_t*
 }
 void launch_vel_residual(const Params& P, cudaStream_t st, const float* Dv, const float* u, const float* uI,
                          double* part, double* out) {
-    WF_LAUNCH(k_vel_residual, Dv, u, uI, part);
+    WF_LAUNCH_SUMS(k_vel_residual, Dv, u, uI, part);
     WF_COUNT_LAUNCH();
     k_sum_partials<<<1, 1024, 0, st>>>(part, cell_grid_blocks(P), out);
 }
 void launch_pres_residual(const Params& P, cudaStream_t st, const float* Dp, const float* pc, const float* pcL,
                           double* part, double* out) {
-    WF_LAUNCH(k_pres_residual, Dp, pc, pcL, part);
+    WF_LAUNCH_SUMS(k_pres_residual, Dp, pc, pcL, part);
     WF_COUNT_LAUNCH();
     k_sum_partials<<<1, 1024, 0, st>>>(part, cell_grid_blocks(P), out);
 }
 void launch_mass_imbalance(const Params& P, const Bnd& B, cudaStream_t st, const uint8_t* fl, const float* u,
                            double* part, double* out) {
-    WF_LAUNCH(k_mass_imbalance, B, fl, u, part);
+    WF_LAUNCH_SUMS(k_mass_imbalance, B, fl, u, part);
     WF_COUNT_LAUNCH();
     k_sum_partials<<<1, 1024, 0, st>>>(part, cell_grid_blocks(P), out);
 }

@@ -744,16 +744,6 @@ __global__ void k_flush_read(const float4* __restrict__ buf, size_t n, float* __
     if (acc == 1.2345f) sink[0] = acc;  // keeps the loads alive
 }
 
-dim3 blk() { return dim3(32, 4, 2); }
-dim3 grd(const Params& P) {
-    dim3 b = blk();
-    return dim3((P.nx + b.x - 1) / b.x, (P.ny + b.y - 1) / b.y, (P.nz + b.z - 1) / b.z);
-}
-dim3 grd4(const Params& P) {
-    const dim3 b = blk();
-    return dim3((P.nx / 4 + b.x - 1) / b.x, (P.ny + b.y - 1) / b.y, (P.nz + b.z - 1) / b.z);
-}
-
 void vel_coef(wf_solver* h) {
     const Params& P = h->P;
     const size_t N = P.N;
@@ -767,7 +757,7 @@ void vel_coef(wf_solver* h) {
         return;
     }
     WF_COUNT_LAUNCH();
-    k_vel_coef<<<grd(P), blk(), 0, h->st>>>(P, h->fl, h->vb[h->iT], h->eddy, h->face, h->Dv, h->vcoef,
+    k_vel_coef<<<cells_grid(P), cells_block(P), 0, h->st>>>(P, h->fl, h->vb[h->iT], h->eddy, h->face, h->Dv, h->vcoef,
                                             h->vcoef + 6 * N);
     h->id_gen = h->d_gen;  // vcoef + 6N now holds 1/D of the current D
 }
@@ -775,9 +765,7 @@ void vel_coef(wf_solver* h) {
 // Block of the four-cell momentum sweep: the handle's tile shape (256
 // threads, x threads cover four cells each).
 dim3 vblk(const wf_solver* h) { return dim3(h->vel_blk[0], h->vel_blk[1], h->vel_blk[2]); }
-dim3 grd4(const Params& P, dim3 b) {
-    return dim3((P.nx / 4 + b.x - 1) / b.x, (P.ny + b.y - 1) / b.y, (P.nz + b.z - 1) / b.z);
-}
+dim3 grd4(const Params& P, dim3 b) { return grid_for(P.nx / 4, P.ny, P.nz, b); }
 
 void launch_vel_sweep_fast(wf_solver* h, const float* src, float* dst) {
     const Params& P = h->P;
@@ -789,7 +777,7 @@ void launch_vel_sweep_fast(wf_solver* h, const float* src, float* dst) {
         launch_chained(k_vel_sweep4<false>, grd4(P, vblk(h)), vblk(h), h->st, h->pdl != 0, P,
                        (const float*)h->vcoef, (const float*)(h->vcoef + 6 * N), (const float*)h->bv, src, dst);
     } else {
-        k_vel_sweep1<false><<<grd(P), blk(), 0, h->st>>>(P, h->vcoef, h->vcoef + 6 * N, h->bv, src, dst);
+        k_vel_sweep1<false><<<cells_grid(P), cells_block(P), 0, h->st>>>(P, h->vcoef, h->vcoef + 6 * N, h->bv, src, dst);
     }
 }
 
@@ -804,12 +792,12 @@ const float* pres_coef(wf_solver* h, bool piso) {
     const float* iDc = h->id_gen == h->d_gen ? h->vcoef + 6 * N : nullptr;
     if (h->c3_gen != h->d_gen) {  // c_E, c_N, c_U depend on D only
         WF_COUNT_LAUNCH();
-        k_pres_coef<<<grd(P), blk(), 0, h->st>>>(P, h->fl, h->Dv, iDc, c3);
+        k_pres_coef<<<cells_grid(P), cells_block(P), 0, h->st>>>(P, h->fl, h->Dv, iDc, c3);
         h->c3_gen = h->d_gen;
     }
     WF_COUNT_LAUNCH();
     if (piso) {
-        k_piso_pre<<<grd(P), blk(), 0, h->st>>>(P, h->fl, h->Dv, iDc, h->aodu, ainv, rhs);
+        k_piso_pre<<<cells_grid(P), cells_block(P), 0, h->st>>>(P, h->fl, h->Dv, iDc, h->aodu, ainv, rhs);
     } else {
         launch_inv(P, h->st, h->fl, h->Dp, ainv);
     }
@@ -820,7 +808,7 @@ void launch_pres_sweep_fast(wf_solver* h, const float* rhs, const float* src, fl
     const Params& P = h->P;
     const size_t N = P.N;
     WF_COUNT_LAUNCH();
-    k_pres_sweep1<<<grd(P), blk(), 0, h->st>>>(P, h->pcoef, h->pcoef + 3 * N, rhs, src, dst);
+    k_pres_sweep1<<<cells_grid(P), cells_block(P), 0, h->st>>>(P, h->pcoef, h->pcoef + 3 * N, rhs, src, dst);
 }
 
 }  // namespace
@@ -1274,20 +1262,20 @@ void launch_pres_stack(const Params& P, cudaStream_t st, int sms, const float* c
 void launch_vel_coef_ptr(const Params& P, cudaStream_t st, const uint8_t* fl, const float* uT, const float* eddy,
                          const float* face, const float* Dv, float* A, float* iD) {
     WF_COUNT_LAUNCH();
-    k_vel_coef<<<grd(P), blk(), 0, st>>>(P, fl, uT, eddy, face, Dv, A, iD);
+    k_vel_coef<<<cells_grid(P), cells_block(P), 0, st>>>(P, fl, uT, eddy, face, Dv, A, iD);
 }
 void launch_vel_sweep1_ptr(const Params& P, cudaStream_t st, const float* A, const float* iD, const float* bv,
                            const float* ui, float* uo) {
     WF_COUNT_LAUNCH();
     if (vec4_ok(P, A, iD, bv, ui, uo))
-        k_vel_sweep4<true><<<grd4(P), blk(), 0, st>>>(P, A, iD, bv, ui, uo);
+        k_vel_sweep4<true><<<grd4(P, groups_block(P)), groups_block(P), 0, st>>>(P, A, iD, bv, ui, uo);
     else
-        k_vel_sweep1<true><<<grd(P), blk(), 0, st>>>(P, A, iD, bv, ui, uo);
+        k_vel_sweep1<true><<<cells_grid(P), cells_block(P), 0, st>>>(P, A, iD, bv, ui, uo);
 }
 void launch_pres_coef_ptr(const Params& P, cudaStream_t st, const uint8_t* fl, const float* Dv, const float* iD,
                           float* c3) {
     WF_COUNT_LAUNCH();
-    k_pres_coef<<<grd(P), blk(), 0, st>>>(P, fl, Dv, iD, c3);
+    k_pres_coef<<<cells_grid(P), cells_block(P), 0, st>>>(P, fl, Dv, iD, c3);
 }
 void launch_inv_ptr(const Params& P, cudaStream_t st, const uint8_t* fl, const float* Dp, float* ainv) {
     WF_COUNT_LAUNCH();
@@ -1296,7 +1284,7 @@ void launch_inv_ptr(const Params& P, cudaStream_t st, const uint8_t* fl, const f
 void launch_piso_pre_ptr(const Params& P, cudaStream_t st, const uint8_t* fl, const float* Dv, const float* iD,
                          const float* aodu, float* ainv, float* rhs) {
     WF_COUNT_LAUNCH();
-    k_piso_pre<<<grd(P), blk(), 0, st>>>(P, fl, Dv, iD, aodu, ainv, rhs);
+    k_piso_pre<<<cells_grid(P), cells_block(P), 0, st>>>(P, fl, Dv, iD, aodu, ainv, rhs);
 }
 
 
