@@ -36,6 +36,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <iterator>
 
 #include "wf_kernels.cuh"
 #include "wf_resident.cuh"
@@ -164,11 +165,34 @@ struct Links {
 };
 // Halo cells a thread fetches at most in the momentum loop of R cells a thread.
 __host__ __device__ constexpr int fetch_max(int R) { return R <= 4 ? 1 : 2; }
+// Halo cell e of the E, W, N, S side: its box coordinates, the box that owns it
+// (-1: outside the domain) and its place t on that box's rim.
+__device__ __forceinline__ int halo_cell(const Box& b, const ResPlan& pl, int e, int& t, int& hx, int& hy) {
+    const int bx = pl.bx, by = pl.by, ix = b.id % pl.px, iy = (b.id / pl.px) % pl.py;
+    if (e < by) {
+        hx = bx; hy = e;
+        t = by + e;
+        return ix + 1 < pl.px ? b.id + 1 : -1;
+    }
+    if (e < 2 * by) {
+        hx = -1; hy = e - by;
+        t = hy;
+        return ix > 0 ? b.id - 1 : -1;
+    }
+    if (e < 2 * by + bx) {
+        hx = e - 2 * by; hy = by;
+        t = hx == bx - 1 ? 0 : hx == 0 ? by : 2 * by + bx - 2 + hx - 1;
+        return iy + 1 < pl.py ? b.id + pl.px : -1;
+    }
+    hx = e - 2 * by - bx; hy = -1;
+    t = hx == bx - 1 ? by - 1 : hx == 0 ? 2 * by - 1 : 2 * by + hx - 1;
+    return iy > 0 ? b.id - pl.px : -1;
+}
 // `groups`: planes whose halo cells are fetched by different threads.
 __device__ __forceinline__ Links make_links(const Box& b, const ResPlan& pl, bool own, int groups) {
     Links l;
     const int tid = threadIdx.x, mine = b.id * b.slots;
-    const int ix = b.id % pl.px, iy = (b.id / pl.px) % pl.py, iz = b.id / (pl.px * pl.py);
+    const int iz = b.id / (pl.px * pl.py);
     l.se = l.su = l.sd = l.ru = l.rd = l.re = -1;
     l.he = 0;
     const int G = groups, g = tid / (b.rim + 4), e = tid % (b.rim + 4);
@@ -187,27 +211,8 @@ __device__ __forceinline__ Links make_links(const Box& b, const ResPlan& pl, boo
             l.rd = (b.id - layer) * b.slots + top + tid;
         }
     }
-    // halo cell e of the E, W, N, S side and the rim thread of the neighbour
-    // box that owns it
-    const int bx = pl.bx, by = pl.by;
-    int from = -1, t = 0, hx = 0, hy = 0;
-    if (e < by) {
-        if (ix + 1 < pl.px) from = b.id + 1;
-        hx = bx; hy = e;
-        t = by + e;
-    } else if (e < 2 * by) {
-        if (ix > 0) from = b.id - 1;
-        hx = -1; hy = e - by;
-        t = hy;
-    } else if (e < 2 * by + bx) {
-        if (iy + 1 < pl.py) from = b.id + pl.px;
-        hx = e - 2 * by; hy = by;
-        t = hx == bx - 1 ? 0 : hx == 0 ? by : 2 * by + bx - 2 + hx - 1;
-    } else {
-        if (iy > 0) from = b.id - pl.px;
-        hx = e - 2 * by - bx; hy = -1;
-        t = hx == bx - 1 ? by - 1 : hx == 0 ? 2 * by - 1 : 2 * by + hx - 1;
-    }
+    int t, hx, hy;
+    const int from = halo_cell(b, pl, e, t, hx, hy);
     l.he = (hy + 1) * b.sx + hx + 1 + g * plane_of(pl.bz);
     if (from >= 0 && l.rn > 0) l.re = from * b.slots + t + g * b.rim;
     return l;
@@ -492,52 +497,52 @@ struct VelArgs {
     size_t half;
     unsigned* ctl;
     int* status;
+    float* stream;   // k_res_vel_wide: the words read in every sweep
 };
 
 // receive() for three components, CS floats apart in the shared box.  Every
-// thread takes a share of the x / y halo, so that one trip fetches it (a rim
-// thread's R packets of four words do not fit beside the coefficients; the
-// pressure loop, whose rim threads hold theirs, lost 5 % by it).  The share is
-// one packet up to R = 4 and two above, fixed at compile time: shares of up to
-// four behind a runtime count cost registers and a branch each.  us a sweep, rim
-// threads alone / up to four / now: 64 x 32 x 48 1.58 / 1.38 / 1.30, 72 x 40 x 72
-// - / 1.61 / 1.55, 100 x 50 x 100 3.72 / 3.38 / 2.96.
-template <int R>
+// thread takes a share of the x / y halo, planes g, g + G, ..., so that one trip
+// fetches it (a rim thread's R packets of four words do not fit beside the
+// coefficients; the pressure loop, whose rim threads hold theirs, lost 5 % by it).
+// The share's limit F is fixed at compile time (one packet up to R = 4 and two
+// above in k_res_vel): shares of up to four behind a runtime count cost registers
+// and a branch each.  us a sweep, rim threads alone / up to four / now: 64 x 32 x
+// 48 1.58 / 1.38 / 1.30, 72 x 40 x 72 - / 1.61 / 1.55, 100 x 50 x 100 3.72 / 3.38 /
+// 2.96.
+template <int F, int CS>
 __device__ __forceinline__ bool receive3(const Links& l, float* v, const Packet3* pk, unsigned ep, float hu[3],
                                          float hd[3]) {
-    constexpr int F = fetch_max(R), CS = R * plane_of(R);
-    const bool nu = l.ru >= 0, nd = l.rd >= 0, ne = l.re >= 0;
-    const Packet3 *pu = pk + (nu ? l.ru : 0), *pd = pk + (nd ? l.rd : 0), *pe = pk + (ne ? l.re : 0);
-    const int second = F > 1 && l.rn > 1 ? l.rstep : 0;
+    const bool nu = l.ru >= 0, nd = l.rd >= 0;
+    const Packet3 *pu = pk + (nu ? l.ru : 0), *pd = pk + (nd ? l.rd : 0);
+    // (the exception saves registers where F is 4: 6.97 -> 6.67 us on 149 x 61 x 103)
+    auto need = [&](int q) { return l.re >= 0 && ((F > 3 && q == 0) || q < l.rn); };
     Packet3 w[F], wu, wd;
     int left = kRounds;
     bool ok;
     do {
         wu = get3(pu);
         wd = get3(pd);
-        w[0] = get3(pe);
-        if (F > 1) w[F - 1] = get3(pe + second);
+#pragma unroll
+        for (int q = 0; q < F; ++q) w[q] = get3(pk + (need(q) ? l.re + q * l.rstep : 0));
         ok = (!nu || (unsigned)(wu.hi >> 32) == ep) && (!nd || (unsigned)(wd.hi >> 32) == ep);
-        ok = ok && (!ne || ((unsigned)(w[0].hi >> 32) == ep && (unsigned)(w[F - 1].hi >> 32) == ep));
-    } while (!__all_sync(0xffffffffu, ok) && --left);
-    if (left == 0) return false;
+#pragma unroll
+        for (int q = 0; q < F; ++q) ok = ok && (!need(q) || (unsigned)(w[q].hi >> 32) == ep);
+    } while (!__all_sync(0xffffffffu, ok) && --left > 0);
+    if (left <= 0) return false;
     hu[0] = nu ? __uint_as_float((unsigned)wu.lo) : 0.f;
     hu[1] = nu ? __uint_as_float((unsigned)(wu.lo >> 32)) : 0.f;
     hu[2] = nu ? __uint_as_float((unsigned)wu.hi) : 0.f;
     hd[0] = nd ? __uint_as_float((unsigned)wd.lo) : 0.f;
     hd[1] = nd ? __uint_as_float((unsigned)(wd.lo >> 32)) : 0.f;
     hd[2] = nd ? __uint_as_float((unsigned)wd.hi) : 0.f;
-    if (ne) {
-        // a thread with one halo cell fetches and writes it twice
-        const int at[2] = {l.he, l.he + (second ? l.hstep : 0)};
 #pragma unroll
-        for (int q = 0; q < F; ++q) {
-            float* o = v + at[q];
+    for (int q = 0; q < F; ++q)
+        if (need(q)) {
+            float* o = v + l.he + q * l.hstep;
             o[0] = __uint_as_float((unsigned)w[q].lo);
             o[CS] = __uint_as_float((unsigned)(w[q].lo >> 32));
             o[2 * CS] = __uint_as_float((unsigned)w[q].hi);
         }
-    }
     return true;
 }
 
@@ -671,7 +676,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
 #pragma unroll
                 for (int r = 0; r < R; ++r) cur[c * CS + r * PS] = u[c][r];
         }
-        if (gridDim.x > 1) bad = !receive3<R>(l, sm, pk, ep, hu, hd);
+        if (gridDim.x > 1) bad = !receive3<fetch_max(R), CS>(l, sm, pk, ep, hu, hd);
         if (__syncthreads_or(bad)) break;
         Packet3* t = pk;
         pk = pk_next;
@@ -689,10 +694,243 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
     epoch_end(a.ctl, base, (unsigned)a.n + 1u);
 }
 
+// ------------------------------------------- momentum, many cells a thread
+// Above 8 cells a thread neither the registers nor the shared memory hold the
+// twelve coefficient words and three values of a cell.  Here the six A_f stay in
+// registers, the iterate in two compact boxes, and of the other six words (1/D and
+// b) NR more in registers and NS in shared memory; the rest is read from L2 in
+// every sweep, from a copy laid out by thread, a plane ahead of its use.
+// Columns go to threads row by row.  A plane has by + 2 rows of bx words, its E
+// and W halo columns behind them: a warp's columns are consecutive words whatever
+// rows they lie in, and only the lanes on an x edge look elsewhere.
+// What bounds it: the shared-memory reads (five a cell and component) and the
+// streamed words while it computes, then a halo trip of 33 KB a box.  Measured,
+// us a sweep: 4.7 on 128 x 64 x 96 (3.1 without the exchange, 4.1 without the
+// streamed words), 6.7 on 149 x 61 x 103, against 5.6 and 11 for one sweep a
+// launch, which moves all 82 bytes of a cell through L2.  Halo cells fetched
+// while the planes are computed, with or without waiting, cost 0.2 us for each
+// packet of a thread; all at the end is the fastest.  E and W halo columns
+// packed without regard to banks cost 0.35 us on the first.
+template <int R> struct Wide;
+template <> struct Wide<10> { static constexpr int PS = 640, NR = 1, NS = 3; };
+template <> struct Wide<12> { static constexpr int PS = 608, NR = 0, NS = 2; };
+template <> struct Wide<14> { static constexpr int PS = 576, NR = 0, NS = 1; };
+template <> struct Wide<15> { static constexpr int PS = 576, NR = 0, NS = 0; };
+constexpr int wide_plane(int R) {
+    return R == 10 ? Wide<10>::PS : R == 12 ? Wide<12>::PS : R == 14 ? Wide<14>::PS : Wide<15>::PS;
+}
+constexpr int wide_streamed(int R) {
+    return 6 - (R == 10 ? Wide<10>::NR + Wide<10>::NS : R == 12 ? Wide<12>::NR + Wide<12>::NS
+                : R == 14 ? Wide<14>::NR + Wide<14>::NS : Wide<15>::NR + Wide<15>::NS);
+}
+template <int R> constexpr size_t wide_smem() {
+    return (6 * (size_t)Wide<R>::PS * R + (size_t)Wide<R>::NS * R * NT) * sizeof(float);
+}
+static_assert(wide_smem<10>() <= kSmemMax && wide_smem<12>() <= kSmemMax && wide_smem<14>() <= kSmemMax &&
+              wide_smem<15>() <= kSmemMax, "boxes exceed the shared memory of one block");
+// The x / y halo of kGroup planes is fetched at once, by as many threads.
+constexpr int kGroup = 4;
+// Places of the E and W halo cells of row ly: in the bank of the word that the
+// lane would read if its row went on, so that a warp's 32 reads stay in 32
+// banks.  The rows' banks repeat after 32 / gcd(bx, 32) rows; with an even bx the
+// E cells lie in even banks and the W cells in odd ones.
+struct Edges {
+    int e, w, period, bx;
+    __host__ __device__ explicit Edges(const ResPlan& p) : bx(p.bx) {
+        const int low = p.bx & -p.bx;
+        period = 32 / (low < 32 ? low : 32);
+        e = (p.bx * (p.by + 2) + 31) / 32 * 32;
+        w = e + (p.bx & 1 ? (p.by + period - 1) / period * 32 : 0);
+    }
+    __host__ __device__ int east(int ly) const { return e + ly / period * 32 + ((ly + 2) * bx & 31); }
+    __host__ __device__ int west(int ly) const { return w + ly / period * 32 + ((ly + 1) * bx + 31 & 31); }
+    __host__ __device__ int words(int by) const { return w + (by + period - 1) / period * 32; }
+};
+
+__device__ __forceinline__ float ld_stream(const float* p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
+template <int R>
+__global__ void __launch_bounds__(NT, 1) k_res_vel_wide(const __grid_constant__ VelArgs a) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr int PS = Wide<R>::PS, CS = R * PS, BUF = 3 * CS;      // plane, component, box
+    constexpr int NR = Wide<R>::NR, NS = Wide<R>::NS, S = 6 - NR - NS;
+    const unsigned base = epoch_begin(a.ctl);
+    const Box b = make_box(a.pl);
+    float* priv = sm + 2 * BUF;                                     // [NS][R][NT]
+    const int tid = threadIdx.x, bx = a.pl.bx, by = a.pl.by, cols = bx * by;
+    const int sxy = a.nx * a.ny;
+    const size_t N = (size_t)sxy * a.nz;
+    const bool own = tid < cols;
+    const int lx = own ? tid % bx : 0, ly = own ? tid / bx : 0;
+    const int x = b.x0 + lx, y = b.y0 + ly;
+    const bool inxy = own && x < a.nx && y < a.ny;
+    const int i0 = inxy ? (b.z0 * a.ny + y) * a.nx + x : 0;
+    const Edges edges(a.pl);
+    const int o0 = (ly + 1) * bx + lx;
+    const int oE = lx == bx - 1 ? edges.east(ly) : o0 + 1, oW = lx == 0 ? edges.west(ly) : o0 - 1;
+    // packets: as in make_links, with the columns in row order
+    Links l;
+    l.se = l.su = l.sd = l.ru = l.rd = l.re = -1;
+    {
+        const int iz = b.id / (a.pl.px * a.pl.py), layer = a.pl.px * a.pl.py;
+        const int mine = b.id * b.slots, top = R * b.rim;
+        if (own) {
+            const bool rim = lx == 0 || lx == bx - 1 || ly == 0 || ly == by - 1;
+            const int t = lx == bx - 1 ? ly : lx == 0 ? by + ly : 2 * by + (ly == by - 1 ? 0 : bx - 2) + lx - 1;
+            if (rim && layer > 1) l.se = mine + t;
+            if (iz + 1 < a.pl.pz) {
+                l.su = mine + top + tid;
+                l.ru = (b.id + layer) * b.slots + top + cols + tid;
+            }
+            if (iz > 0) {
+                l.sd = mine + top + cols + tid;
+                l.rd = (b.id - layer) * b.slots + top + tid;
+            }
+        }
+    }
+    const int g = tid / (b.rim + 4), e = tid % (b.rim + 4);
+    int ht, hx, hy;
+    const int from = halo_cell(b, a.pl, e, ht, hx, hy);
+    l.he = hx == bx ? edges.east(hy) : hx < 0 ? edges.west(hy) : (hy + 1) * bx + hx;
+    hx += b.x0;
+    hy += b.y0;
+    // the input iterate with its halo, zero outside the domain
+    for (int o = tid; o < 2 * BUF; o += NT) sm[o] = 0.f;
+    __syncthreads();
+    float hu[3] = {0.f, 0.f, 0.f}, hd[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (inxy && b.z0 + r < a.nz) sm[c * CS + r * PS + o0] = __ldg(a.uin + c * N + i0 + r * sxy);
+        if (inxy && b.z0 > 0) hd[c] = __ldg(a.uin + c * N + i0 - sxy);
+        if (inxy && b.z0 + R < a.nz) hu[c] = __ldg(a.uin + c * N + i0 + R * sxy);
+    }
+    if (g == 0 && hx >= 0 && hx < a.nx && hy >= 0 && hy < a.ny) {
+        for (int c = 0; c < 3; ++c)
+            for (int r = 0; r < R && b.z0 + r < a.nz; ++r)
+                sm[c * CS + r * PS + l.he] = __ldg(a.uin + c * N + (size_t)(b.z0 + r) * sxy + hy * a.nx + hx);
+    }
+    l.rstep = kGroup * b.rim;
+    l.hstep = kGroup * PS;
+    l.rn = g < kGroup ? (R - 1 - g) / kGroup + 1 : 0;
+    l.he += g * PS;
+    if (from >= 0 && l.rn > 0) l.re = from * b.slots + ht + g * b.rim;
+    // the column's coefficients: words 0..5 are 1/D_x, b_x, b_y, b_z, 1/D_y, 1/D_z
+    // (1/D is 0 on solid cells, whose b is not theirs)
+    float A[6][R], wr[NR > 0 ? NR : 1][R];
+    float* str = a.stream + (size_t)b.id * (R * S * NT) + tid;      // [R][S][NT] of this box
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = i0 + r * sxy;
+        const bool in = inxy && b.z0 + r < a.nz;
+#pragma unroll
+        for (int f = 0; f < 6; ++f) A[f][r] = in ? __ldg(a.A + f * N + i) : 0.f;
+        const float d0 = in ? __ldg(a.iD + i) : 0.f;
+        const bool fluid = d0 != 0.f;
+#pragma unroll
+        for (int w = 0; w < 6; ++w) {
+            const float* src = w == 0 ? a.iD : w < 4 ? a.bv + (w - 1) * N : a.iD + (w - 3) * N;
+            const float v = w == 0 ? d0 : fluid ? __ldg(src + i) : 0.f;
+            if (w < NR) wr[w < NR ? w : 0][r] = v;
+            else if (w < NR + NS) priv[((w - NR) * R + r) * NT + tid] = v;
+            else str[(r * S + w - NR - NS) * NT] = v;
+        }
+    }
+    float next[S > 0 ? S : 1];
+    auto fetch = [&](int r) {
+#pragma unroll
+        for (int s = 0; s < S; ++s) next[s] = ld_stream(str + (r * S + s) * NT);
+    };
+    // One sweep from the box `cu`; plane(r, old, new, 1/D_x) takes the results of
+    // plane r.
+    auto sweep = [&](const float* cu, auto plane) {
+        float cen[3], bel[3];
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const int r = j == 0 ? R - 1 : j - 1;
+            float w[6];
+#pragma unroll
+            for (int s = 0; s < S; ++s) w[NR + NS + s < 6 ? NR + NS + s : 0] = next[s];
+            if (j + 1 < R) fetch(j);
+#pragma unroll
+            for (int q = 0; q < NR + NS; ++q) w[q] = q < NR ? wr[q < NR ? q : 0][r] : priv[((q - NR) * R + r) * NT + tid];
+            float v[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int k = c * CS + r * PS;
+                if (j < 2) {
+                    cen[c] = cu[o0 + k];
+                    bel[c] = j == 0 ? cu[o0 + k - PS] : hd[c];
+                }
+                const float up = j == 0 ? hu[c] : cu[o0 + k + PS];
+                // in the order of k_vel_sweep4
+                float acc = A[0][r] * cu[oE + k];
+                acc += A[1][r] * cu[oW + k];
+                acc += A[2][r] * cu[o0 + bx + k];
+                acc += A[3][r] * cu[o0 - bx + k];
+                acc += A[4][r] * up;
+                acc += A[5][r] * bel[c];
+                v[c] = w[c == 0 ? 0 : 3 + c] * (acc + w[1 + c]);
+                bel[c] = cen[c];
+                if (j > 0) cen[c] = up;
+            }
+            plane(r, bel, v, w[0]);
+        }
+    };
+    __syncthreads();
+    fetch(R - 1);
+    Packet3 *pk = a.pk, *pk_next = a.pk + a.half;
+    unsigned ep = base;
+    int at = 0;
+    bool bad = false;
+    for (int k = 1; k < a.n; ++k) {
+        ++ep;
+        const float* cu = sm + at;
+        float* nb = sm + (BUF - at);
+        sweep(cu, [&](int r, const float*, const float* v, float) {
+            if (own) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) nb[o0 + c * CS + r * PS] = v[c];
+            }
+            if (l.se >= 0) put3(pk + l.se + r * b.rim, v[0], v[1], v[2], ep);
+            if (r == 0 && l.sd >= 0) put3(pk + l.sd, v[0], v[1], v[2], ep);
+            if (r == R - 1 && l.su >= 0) put3(pk + l.su, v[0], v[1], v[2], ep);
+        });
+        fetch(R - 1);
+        if (gridDim.x > 1) bad = !receive3<(R + kGroup - 1) / kGroup, CS>(l, nb, pk, ep, hu, hd);
+        if (__syncthreads_or(bad)) break;
+        Packet3* t = pk;
+        pk = pk_next;
+        pk_next = t;
+        at = BUF - at;
+    }
+    if (ep != base + (unsigned)a.n - 1u || __syncthreads_or(bad)) bad = true;
+    if (bad) {
+        if (tid == 0 && a.status) atomicExch(a.status, 1);
+    } else {
+        sweep(sm + at, [&](int r, const float* old, const float* v, float d0) {
+            if (inxy && b.z0 + r < a.nz && d0 != 0.f) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    a.uout[c * N + i0 + r * sxy] = v[c];
+                    if (a.uprev) a.uprev[c * N + i0 + r * sxy] = old[c];
+                }
+            }
+        });
+    }
+    epoch_end(a.ctl, base, (unsigned)a.n + 1u);
+}
+
 // Cells per thread the kernels are built for.
 constexpr int kPresR[] = {2, 3, 4, 6, 8, 10, 12, 14, 16};
 constexpr int kNuPresR[] = {2, 3, 4, 6, 8};
 constexpr int kVelR[] = {2, 3, 4, 6, 8};
+constexpr int kVelWideR[] = {10, 12, 14, 15};
 
 using PresKernel = void (*)(const PresArgs);
 template <Form F, bool STACK>
@@ -725,6 +963,10 @@ VelKernel vel_kernel(int R) {
         case 4: return k_res_vel<4>;
         case 6: return k_res_vel<6>;
         case 8: return k_res_vel<8>;
+        case 10: return k_res_vel_wide<10>;
+        case 12: return k_res_vel_wide<12>;
+        case 14: return k_res_vel_wide<14>;
+        case 15: return k_res_vel_wide<15>;
         default: return nullptr;
     }
 }
@@ -734,11 +976,20 @@ VelKernel vel_kernel(int R) {
 // 1.45-1.67 with 8 in 4 to 8 warps, 1.75 in 16 warps, 2.3 with 12, 2.6-2.9 with
 // 14, 3.4 with 16: the cells of a thread weigh most (a warp works through
 // them one after another), then the warps, then the halo.
+// loop: whose limits the split has to keep.
 // shared: beside other cases' loops the product of a sweep's time and the
 // multiprocessors it holds counts instead, so that as many loops as possible
 // run at once.
+enum class Loop { kPres, kVel, kVelWide };
+bool fits(const ResPlan& pl, Loop loop) {
+    if (rim_of(pl) + 4 > NT) return false;
+    if (loop == Loop::kVelWide)
+        return pl.bx * pl.by <= NT && Edges(pl).words(pl.by) <= wide_plane(pl.bz) && kGroup * (rim_of(pl) + 4) <= NT;
+    return inner0_of(pl) + inner_of(pl) <= NT && (pl.bx + kPad) * (pl.by + 2) <= plane_of(pl.bz) &&
+           (loop == Loop::kPres || fetches_of(pl) <= fetch_max(pl.bz));
+}
 template <size_t M>
-ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], bool momentum = false, bool shared = false) {
+ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], Loop loop = Loop::kPres, bool shared = false) {
     ResPlan best;
     double cost = 1e30;
     sms = std::min(sms, kMaxBoxes);
@@ -753,9 +1004,7 @@ ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], bool momentum = 
                 ResPlan pl;
                 pl.bx = bx; pl.by = by; pl.bz = R;
                 pl.px = px; pl.py = py; pl.pz = pz;
-                if (inner0_of(pl) + inner_of(pl) > NT || (bx + kPad) * (by + 2) > plane_of(R) ||
-                    rim_of(pl) + 4 > NT || (momentum && fetches_of(pl) > fetch_max(R)))
-                    continue;
+                if (!fits(pl, loop)) continue;
                 const double halo = 2.0 * ((px > 1 ? by * R : 0) + (py > 1 ? bx * R : 0) + (pz > 1 ? bx * by : 0));
                 double c = R * (60.0 + 0.6 * (inner0_of(pl) / 32 + (inner_of(pl) + 31) / 32)) + 0.03 * halo;
                 if (shared) c = (500.0 + c) * pl.boxes();
@@ -767,6 +1016,19 @@ ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], bool momentum = 
         }
     }
     return best;
+}
+// Words of the momentum loop's streamed coefficients.
+size_t streamed(const ResPlan& p) {
+    return p.bz > kVelR[std::size(kVelR) - 1] ? (size_t)p.boxes() * p.bz * wide_streamed(p.bz) * NT : 0;
+}
+size_t vel_bytes(int R) {
+    switch (R) {
+        case 10: return wide_smem<10>();
+        case 12: return wide_smem<12>();
+        case 14: return wide_smem<14>();
+        case 15: return wide_smem<15>();
+        default: return vel_smem(R);
+    }
 }
 size_t packets(const ResPlan& p) {
     return p.bz > 0 ? (size_t)p.boxes() * slots_of(p) : 0;
@@ -809,9 +1071,10 @@ int resident_setup(const Resident& r) {
 void resident_plan(const Params& P, int sms, Resident* r) {
     r->pres = make_plan(P, sms, kPresR);
     r->nupres = make_plan(P, sms, kNuPresR);
-    r->vel = make_plan(P, sms, kVelR, true);
-    r->pres_shared = make_plan(P, sms, kPresR, false, true);
-    r->vel_shared = make_plan(P, sms, kVelR, true, true);
+    r->vel = make_plan(P, sms, kVelR, Loop::kVel);
+    if (r->vel.bz == 0) r->vel = make_plan(P, sms, kVelWideR, Loop::kVelWide);
+    r->pres_shared = make_plan(P, sms, kPresR, Loop::kPres, true);
+    r->vel_shared = make_plan(P, sms, kVelR, Loop::kVel, true);
 }
 
 void resident_alloc(Resident* r, cudaStream_t st) {
@@ -821,13 +1084,14 @@ void resident_alloc(Resident* r, cudaStream_t st) {
     const size_t np = 2 * std::max({packets(r->pres), packets(r->nupres), packets(r->pres_shared)}),
                  nv = 2 * std::max(packets(r->vel), packets(r->vel_shared));
     if (np + nv == 0 || r->work.pk) return;
-    const size_t bytes = np * sizeof(unsigned long long) + nv * sizeof(Packet3) + 16;
+    const size_t bytes = np * sizeof(unsigned long long) + nv * sizeof(Packet3) + 16 +
+                         streamed(r->vel) * sizeof(float);
     void* pk = nullptr;
     if (cudaMalloc(&pk, bytes) != cudaSuccess) {
         cudaGetLastError();
         return;
     }
-    if (cudaMemsetAsync(pk, 0, bytes, st) != cudaSuccess) {
+    if (cudaMemsetAsync(pk, 0, bytes - streamed(r->vel) * sizeof(float), st) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(pk);
         return;
@@ -835,6 +1099,7 @@ void resident_alloc(Resident* r, cudaStream_t st) {
     r->work.pk = pk;
     r->work.pk3 = static_cast<unsigned long long*>(pk) + np;  // np is even: 16-byte aligned
     r->work.ctl = reinterpret_cast<unsigned*>(static_cast<Packet3*>(r->work.pk3) + nv);
+    r->work.stream = reinterpret_cast<float*>(r->work.ctl + 4);
 }
 
 void resident_free(Resident* r) {
@@ -890,7 +1155,8 @@ cudaError_t launch_res_vel(const Params& P, cudaStream_t st, const ResPlan& pl, 
     a.half = packets(pl);
     a.ctl = w.ctl;
     a.status = status;
-    const cudaError_t e = launch_coop((const void*)vel_kernel(pl.bz), pl.boxes(), vel_smem(pl.bz), st, &a);
+    a.stream = w.stream;
+    const cudaError_t e = launch_coop((const void*)vel_kernel(pl.bz), pl.boxes(), vel_bytes(pl.bz), st, &a);
     if (e == cudaSuccess) WF_COUNT_LAUNCH();
     else cudaGetLastError();
     return e;

@@ -16,11 +16,12 @@ struct ResPlan {
 };
 
 // Device workspace of the loops of one stream: the halo packets of both
-// parities and the epoch words.  One loop at a time may use it.
+// parities, the epoch words and streamed coefficients.  One loop at a time may use it.
 struct ResWork {
     void* pk = nullptr;    // the allocation; 64-bit packets of the pressure loops
     void* pk3 = nullptr;   // 128-bit packets of the momentum loop
     unsigned* ctl = nullptr;
+    float* stream = nullptr;  // coefficients the momentum loop reads in every sweep
 };
 
 // The plans of one handle's loops and their workspace.
