@@ -198,6 +198,7 @@ int do_vel_precompute(wf_solver* h) {
                               h->P.les ? h->bv : nullptr, h->drag, h->Dv, h->bv, A, iD);
     WF_CHECK_LAUNCH();
     h->vcoef_step = coef;
+    if (coef) h->id_gen = h->d_gen;
     return WF_OK;
 }
 
@@ -242,7 +243,7 @@ int do_vel_sweeps(wf_solver* h, int n, bool allow_fast) {
         if (h->nonuniform)  // the pre-compute's A and 1/D (vcoef)
             wf::launch_vel_sweep1_ptr(P, h->st, h->vcoef, h->vcoef + 6 * (size_t)P.N, h->bv, src, h->vb[h->iF]);
         else
-            wf::launch_vel_sweep(P, h->st, h->fl, src, h->vb[h->iT], h->eddy, h->face, h->Dv, h->bv, h->vb[h->iF]);
+            wf::launch_vel_sweep(P, h->st, src, h->vb[h->iT], h->eddy, h->Dv, cur_inv_d(h), h->bv, h->vb[h->iF]);
         WF_CHECK_LAUNCH();
         if (resid && k % h->cfg.vel_res_interval == 0) {
             bool done = false;
@@ -297,7 +298,7 @@ int do_pres_sweeps(wf_solver* h, int n, bool allow_fast) {
         if (h->nonuniform)
             wf::launch_nu_pres_sweep(h, src, h->pcb[h->iPC], k > 0);
         else
-            wf::launch_pres_sweep(P, h->st, h->fl, src, h->Dv, h->Dp, h->bp, h->pcb[h->iPC]);
+            wf::launch_pres_sweep(P, h->st, src, h->Dv, cur_inv_d(h), h->Dp, h->bp, h->pcb[h->iPC]);
         WF_CHECK_LAUNCH();
         h->pc_zero = false;
         bool done = false;
@@ -306,13 +307,16 @@ int do_pres_sweeps(wf_solver* h, int n, bool allow_fast) {
         std::swap(h->iPCL, h->iPC);
         if (!chip) continue;
         const int interval = h->cfg.pres_res_interval;
-        const int m = std::min((k / interval + 1) * interval, n - 1) - k;  // sweeps up to the next check
-        if (m < 2 || !wf::pres_sweeps_on_chip(h, m, coef_done, true)) continue;
-        coef_done = true;
-        k += m;
-        if (k % interval == 0) WF_TRY(pres_converged(h, h->pcb[h->iPC], h->pcb[h->iPCL], &done));
+        for (;;) {
+            const int m = std::min((k / interval + 1) * interval, n - 1) - k;  // sweeps up to the next check
+            if (m < 2 || !wf::pres_sweeps_on_chip(h, m, coef_done, true)) break;
+            coef_done = true;
+            k += m;
+            if (k % interval == 0) WF_TRY(pres_converged(h, h->pcb[h->iPC], h->pcb[h->iPCL], &done));
+            if (done) break;
+            std::swap(h->iPCL, h->iPC);
+        }
         if (done) break;
-        std::swap(h->iPCL, h->iPC);
     }
     std::swap(h->iPCL, h->iPC);
     return WF_OK;

@@ -24,13 +24,13 @@ void launch_les_term(const Params& P, const Bnd& B, cudaStream_t st, const uint8
 void launch_vel_precompute(const Params& P, const Bnd& B, cudaStream_t st, const uint8_t* fl, const float* uT,
                            const float* pr, const float* eddy, const float* face, const float* bles,
                            const float* drag, float* Dv, float* bv, float* A = nullptr, float* iD = nullptr);
-void launch_vel_sweep(const Params& P, cudaStream_t st, const uint8_t* fl, const float* uI, const float* uT,
-                      const float* eddy, const float* face, const float* Dv, const float* bv, float* uo);
+void launch_vel_sweep(const Params& P, cudaStream_t st, const float* uI, const float* uT, const float* eddy,
+                      const float* Dv, const float* iD, const float* bv, float* uo);
 // iD (nullable): cached 1/D of the same D (bit-identical to dividing).
 void launch_pres_precompute(const Params& P, const Bnd& B, cudaStream_t st, const uint8_t* fl, const float* u,
                             const float* pr, const float* Dv, const float* iD, float* Dp, float* bp,
                             float* c3 = nullptr);
-void launch_pres_sweep(const Params& P, cudaStream_t st, const uint8_t* fl, const float* pin, const float* Dv,
+void launch_pres_sweep(const Params& P, cudaStream_t st, const float* pin, const float* Dv, const float* iD,
                        const float* Dp, const float* bp, float* pout);
 void launch_apply_pres(const Params& P, cudaStream_t st, const uint8_t* fl, const float* pc, float* pr);
 void launch_normalize(const Params& P, cudaStream_t st, const uint8_t* fl, float* pr, float* ref);
