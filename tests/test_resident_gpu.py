@@ -59,6 +59,22 @@ def test_loops_outside_a_step(built, n):
     _same(a, b)
 
 
+# two sweeps a halo trip with 2, 3 and 4 cells a thread, boxes of two cells, and
+# boxes that overhang the domain on every axis; odd and even sweep counts
+@pytest.mark.parametrize("grid", [(64, 32, 48), (53, 31, 37), (61, 31, 59), (72, 36, 60), (6, 5, 7)],
+                         ids=lambda g: "%dx%dx%d" % g)
+def test_two_sweeps_a_trip(built, grid):
+    nx, ny, nz = grid
+    case = cases.small_case(nx=nx, ny=ny, nz=nz, seed=nz)
+    a, b = _pair(case)
+    for s in (a, b):
+        s.Step(1)
+        s.op("vel_precompute"); s.op("vel_sweeps", 2); s.op("pres_precompute")
+        for n in (2, 3, 4, 7, 12):
+            s.op("pres_sweeps", n)
+    _same(a, b)
+
+
 @pytest.mark.parametrize("kw", [dict(), dict(log_inflow=True, les=True), dict(nx=15, x_split=(7, 4))],
                          ids=["tunnel", "urban_les", "odd"])
 def test_stretched_mesh_bit_identical(built, kw):

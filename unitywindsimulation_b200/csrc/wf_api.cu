@@ -284,14 +284,14 @@ int do_pres_sweeps(wf_solver* h, int n, bool allow_fast) {
         WF_TRY(wf::pres_sweeps_fast(h, n, /*piso=*/false));
         return WF_OK;
     }
-    if (allow_fast && !resid && n >= 2 && wf::loops_on_chip(h, h->res.nupres) &&
+    if (allow_fast && !resid && n >= 2 && wf::loops_on_chip(h, h->res.nupres_alone()) &&
         wf::pres_sweeps_on_chip(h, n, true, !h->in_step))
         return WF_OK;
     // with residual checks: the sweeps up to the next one on chip, in the
     // sums of the kernels below.  One sweep a launch took 6.5 of the 8.2 ms of
     // a step on 100 x 50 x 100 (400 sweeps, checked every 20).  (The momentum
     // loop has no such form: 12 instead of 7 coefficients a cell do not fit.)
-    const bool chip = allow_fast && resid && wf::loops_on_chip(h, h->nonuniform ? h->res.nupres : h->res.pres);
+    const bool chip = allow_fast && resid && wf::loops_on_chip(h, h->nonuniform ? h->res.nupres_alone() : h->res.pres_alone());
     bool coef_done = false;
     for (int k = 0; k < n; ++k) {
         const float* src = h->pc_zero ? nullptr : h->pcb[h->iPCL];

@@ -477,6 +477,251 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
     epoch_end(a.ctl, base, (unsigned)a.n + 1u);
 }
 
+// ---------------------------------------------- pressure, two sweeps a trip
+// On small grids a sweep is mostly the packets' trip.  Here a box exchanges two
+// layers of cells (and the edges between them) and runs two sweeps on them: the
+// first also on the cells next to the box, which it computes as their owners do,
+// the second on its own cells.
+// A thread holds a column of the box or of the ring around it, with one cell above
+// and below.  Rows of a plane: y = -2 .. by + 1 of bx + 2 words, then the cells two
+// off the x faces; planes z = -2 .. R + 1.  A cell's packet has the cell's place in
+// its box; the table lists the halo cells, their packets and places.
+// Bound by the trip: a pair computes for 0.6 us and waits for 0.9.  Polling takes
+// the bandwidth that the packets need (a round reads 2000 of them a box), so a box
+// waits kPairWait cycles, about a trip, before the first round, and asks only for
+// what is missing after it.  us a sweep, one sweep a trip / pairs polled at once /
+// pairs that wait: 64 x 32 x 48 1.10 / 0.95 / 0.77, 80 x 40 x 40 1.16 / 0.98 / 0.81.
+// It pays while one round fetches the halo (4 cells a thread): at 72 x 40 x 72,
+// 2216 halo cells, 1.21 in either form; and up to 4 cells a thread (with 6 and 8
+// the halo computed twice outgrows the trip: 1.2-1.6).
+constexpr int kPairPlane = 736, kPairFetch = 4;  // words of a plane; halo cells a thread fetches at most
+constexpr int kPairWait = 600;                     // cycles
+constexpr int pair_plane_words(const ResPlan& p) { return (p.bx + 2) * (p.by + 4) + 2 * p.by; }
+__host__ __device__ constexpr int pair_halo(const ResPlan& p) {
+    return 4 * (p.bx * p.by + p.bx * p.bz + p.by * p.bz + p.bx + p.by + p.bz);
+}
+constexpr size_t pair_smem(const ResPlan& p) {
+    return 2 * (size_t)(p.bz + 4) * kPairPlane * sizeof(float) + (size_t)pair_halo(p) * sizeof(int2);
+}
+// Box coordinates of halo cell e.
+__device__ __forceinline__ void pair_cell(const ResPlan& p, int e, int& lx, int& ly, int& lz) {
+    const int bx = p.bx, by = p.by, bz = p.bz;
+    auto side = [](int q, int b) { return q == 0 ? -1 : q == 1 ? -2 : q == 2 ? b : b + 1; };
+    int n = bx * by;
+    if (e < 4 * n) {
+        lz = side(e / n, bz);
+        lx = e % n % bx;
+        ly = e % n / bx;
+        return;
+    }
+    e -= 4 * n;
+    n = bx * bz;
+    if (e < 4 * n) {
+        ly = side(e / n, by);
+        lx = e % n % bx;
+        lz = e % n / bx;
+        return;
+    }
+    e -= 4 * n;
+    n = by * bz;
+    if (e < 4 * n) {
+        lx = side(e % 2 + e / (2 * n) * 2, bx);  // the two layers side by side: one sector
+        ly = e / 2 % by;
+        lz = e / 2 % n / by;
+        return;
+    }
+    e -= 4 * n;
+    auto lo = [](int q, int b) { return q ? b : -1; };
+    if (e < 4 * bx) {
+        lx = e % bx;
+        ly = lo(e / bx & 1, by);
+        lz = lo(e / bx >> 1, bz);
+        return;
+    }
+    e -= 4 * bx;
+    if (e < 4 * by) {
+        ly = e % by;
+        lx = lo(e / by & 1, bx);
+        lz = lo(e / by >> 1, bz);
+        return;
+    }
+    e -= 4 * by;
+    lz = e % bz;
+    lx = lo(e / bz & 1, bx);
+    ly = lo(e / bz >> 1, by);
+}
+
+template <int R, Form F>
+__global__ void __launch_bounds__(NT, 1) k_res_pair(const __grid_constant__ PresArgs a) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr bool NU = F == Form::kStretched;
+    constexpr int PS = kPairPlane, BUF = (R + 4) * PS, E = R + 2;
+    const unsigned base = epoch_begin(a.ctl);
+    const int bx = a.pl.bx, by = a.pl.by, px = a.pl.px, py = a.pl.py, id = blockIdx.x;
+    const int x0 = id % px * bx, y0 = id / px % py * by, z0 = id / (px * py) * R;
+    const int tid = threadIdx.x, w = bx + 2, cells = R * bx * by;
+    const int sxy = a.nx * a.ny;
+    const size_t N = (size_t)sxy * a.nz;
+    float *s0 = sm, *s1 = sm + BUF;
+    int2* tab = reinterpret_cast<int2*>(sm + 2 * BUF);
+    const int H = gridDim.x > 1 ? pair_halo(a.pl) : 0;
+    for (int o = tid; o < 2 * BUF; o += NT) sm[o] = 0.f;
+    __syncthreads();
+    for (int e = tid; e < H; e += NT) {
+        int lx, ly, lz;
+        pair_cell(a.pl, e, lx, ly, lz);
+        const int x = x0 + lx, y = y0 + ly, z = z0 + lz;
+        const int row = lx == -2 ? w * (by + 4) + ly : lx == bx + 1 ? w * (by + 4) + by + ly : (ly + 2) * w + lx + 1;
+        int2 t = make_int2(-1, (lz + 2) * PS + row);
+        if (x >= 0 && x < a.nx && y >= 0 && y < a.ny && z >= 0 && z < a.nz) {
+            const int ox = lx < 0 ? -1 : lx >= bx, oy = ly < 0 ? -1 : ly >= by, oz = lz < 0 ? -1 : lz >= R;
+            t.x = (id + ox + px * (oy + py * oz)) * cells + (lx - ox * bx) + bx * ((ly - oy * by) + by * (lz - oz * R));
+            if (a.pin) s0[t.y] = __ldg(a.pin + ((size_t)z * a.ny + y) * a.nx + x);
+        }
+        tab[e] = t;
+    }
+    const int lx = tid % w - 1, ly = tid / w - 1;
+    const bool ringx = lx < 0 || lx >= bx, ringy = ly < 0 || ly >= by, own = !ringx && !ringy;
+    const int x = x0 + lx, y = y0 + ly;
+    const bool col = ly <= by && !(ringx && ringy) && x >= 0 && x < a.nx && y >= 0 && y < a.ny;
+    const int o = col ? tid + w : w;
+    const int oE = col && lx == bx ? w * (by + 4) + by + ly : o + 1, oW = col && lx < 0 ? w * (by + 4) + ly : o - 1;
+    const int i0 = col ? y * a.nx + x : 0;
+    const int slot = id * cells + ly * bx + lx;
+    const bool edge = own && (lx < 2 || lx >= bx - 2 || ly < 2 || ly >= by - 2);
+    const bool mine = own && col, lo = mine && z0 > 0, hi = mine && z0 + R < a.nz;
+    // coefficients of the column's cells, j = 0 .. R + 1 for z = -1 .. R
+    float cE[E], cW[E], cN[E], cS[E], cU[E], cD[NU ? E : 1], ai[E], rh[E];
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+        const int z = z0 + j - 1;
+        const bool inz = col && z >= 0 && z < a.nz;
+        bool in = inz && (own || (j > 0 && j <= R));
+        const int i = inz ? z * sxy + i0 : 0;
+        if (mine && a.pin && j > 0 && j <= R && inz) s0[o + (j + 1) * PS] = __ldg(a.pin + i);
+        if (NU && in) in = (__ldg(a.nbm + i) & 64u) != 0;  // solid cells hold no coefficients
+        if (NU) {
+            cE[j] = in ? __ldg(a.c + i) : 0.f;
+            cW[j] = in ? __ldg(a.c + N + i) : 0.f;
+            cN[j] = in ? __ldg(a.c + 2 * N + i) : 0.f;
+            cS[j] = in ? __ldg(a.c + 3 * N + i) : 0.f;
+            cU[j] = in ? __ldg(a.c + 4 * N + i) : 0.f;
+            cD[NU ? j : 0] = in ? __ldg(a.c + 5 * N + i) : 0.f;
+        } else {
+            cE[j] = in ? __ldg(a.c + i) : 0.f;
+            cW[j] = in && x > 0 ? __ldg(a.c + i - 1) : 0.f;
+            cN[j] = in ? __ldg(a.c + N + i) : 0.f;
+            cS[j] = in && y > 0 ? __ldg(a.c + N + i - a.nx) : 0.f;
+            cU[j] = inz ? __ldg(a.c + 2 * N + i) : 0.f;
+            if (j == 0) cD[0] = in && z > 0 ? __ldg(a.c + 2 * N + i - sxy) : 0.f;
+        }
+        ai[j] = in ? __ldg(a.ainv + i) : 0.f;
+        rh[j] = in && a.rhs ? __ldg(a.rhs + i) : 0.f;
+    }
+    // cell j of the column from the iterate at s
+    auto cell = [&](const float* s, int j, float up, float below) {
+        const float* q = s + (j + 1) * PS;
+        float acc = F == Form::kPasses ? __fmaf_rn(-cE[j], q[oE], __fmul_rn(-cW[j], q[oW]))
+                                       : __fmaf_rn(-cW[j], q[oW], __fmul_rn(-cE[j], q[oE]));
+        acc = __fmaf_rn(-cN[j], q[o + w], acc);
+        acc = __fmaf_rn(-cS[j], q[o - w], acc);
+        acc = __fmaf_rn(-cU[j], up, acc);
+        acc = __fmaf_rn(-(NU ? cD[NU ? j : 0] : j > 0 ? cU[j > 0 ? j - 1 : 0] : cD[0]), below, acc);
+        return ai[j] * (acc + rh[j]);
+    };
+    // cells first .. last from the iterate at s; all of them before the first
+    // store, so that no load waits for one
+    float v[E];
+    auto sweep = [&](const float* s, int first, int last) {
+        float below = s[o + first * PS], cen = s[o + (first + 1) * PS];
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            if (j < first || j > last) continue;
+            const float up = s[o + (j + 2) * PS];
+            v[j] = cell(s, j, up, below);
+            below = cen;
+            cen = up;
+        }
+    };
+    auto outer = [&]() {
+        sweep(s0, 0, R + 1);
+#pragma unroll
+        for (int j = 0; j < E; ++j)
+            if (j == 0 ? lo : j == R + 1 ? hi : col) s1[o + (j + 1) * PS] = v[j];
+    };
+    __syncthreads();
+    unsigned long long *pk = a.pk, *pk_next = a.pk + a.half;
+    unsigned ep = base;
+    bool bad = false;
+    const int pairs = (a.n - 1) / 2;
+    for (int k = 0; k < pairs; ++k) {
+        ++ep;
+        outer();
+        __syncthreads();
+        if (mine) {
+            sweep(s1, 1, R);
+            unsigned long long* dst = pk + slot;
+#pragma unroll
+            for (int j = 1; j <= R; ++j)
+                if (H > 0 && (R <= 4 || edge || j <= 2 || j >= R - 1)) put(dst + (j - 1) * bx * by, v[j], ep);
+#pragma unroll
+            for (int j = 1; j <= R; ++j) s0[o + (j + 1) * PS] = v[j];
+        }
+        int left = kRounds;
+        if (H > 0) {
+            const long long t0 = clock64();
+            while (clock64() - t0 < kPairWait) {}
+            int2 t[kPairFetch];
+            unsigned long long g[kPairFetch];
+#pragma unroll
+            for (int u = 0; u < kPairFetch; ++u) {
+                t[u] = tid + u * NT < H ? tab[tid + u * NT] : make_int2(-1, 0);
+                g[u] = 0;
+            }
+            bool ok;
+            do {
+                ok = true;
+#pragma unroll
+                for (int u = 0; u < kPairFetch; ++u)
+                    if (t[u].x >= 0 && (unsigned)(g[u] >> 32) != ep) g[u] = get(pk + t[u].x);
+#pragma unroll
+                for (int u = 0; u < kPairFetch; ++u) ok = ok && (t[u].x < 0 || (unsigned)(g[u] >> 32) == ep);
+            } while (!__all_sync(0xffffffffu, ok) && --left > 0);
+#pragma unroll
+            for (int u = 0; u < kPairFetch; ++u)
+                if (t[u].x >= 0) s0[t[u].y] = __uint_as_float((unsigned)g[u]);
+        }
+        if (__syncthreads_or(left <= 0)) {
+            bad = true;
+            break;
+        }
+        unsigned long long* t = pk;
+        pk = pk_next;
+        pk_next = t;
+    }
+    if (bad) {
+        if (tid == 0 && a.status) atomicExch(a.status, 1);
+    } else {
+        const float* from = s0;
+        if (a.n - 2 * pairs == 2) {
+            outer();
+            from = s1;
+            __syncthreads();
+        }
+        if (mine) {
+            sweep(from, 1, R);
+#pragma unroll
+            for (int j = 1; j <= R; ++j)
+                if (z0 + j - 1 < a.nz && ai[j] != 0.f) {
+                    const size_t i = (size_t)(z0 + j - 1) * sxy + i0;
+                    if (a.pprev) a.pprev[i] = from[o + (j + 1) * PS];
+                    if (a.pout) a.pout[i] = v[j];
+                }
+        }
+    }
+    epoch_end(a.ctl, base, (unsigned)a.n + 1u);
+}
+
 // ---------------------------------------------------------------- momentum
 // Sweeps u = (1/D) (sum_f A_f u_f + b) of the three components.  One shared
 // box (a second barrier a sweep separates its readers from its writers: two
@@ -929,6 +1174,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel_wide(const __grid_constant__ 
 // Cells per thread the kernels are built for.
 constexpr int kPresR[] = {2, 3, 4, 6, 8, 10, 12, 14, 16};
 constexpr int kNuPresR[] = {2, 3, 4, 6, 8};
+constexpr int kPairR[] = {2, 3, 4};
 constexpr int kVelR[] = {2, 3, 4, 6, 8};
 constexpr int kVelWideR[] = {10, 12, 14, 15};
 
@@ -953,6 +1199,16 @@ PresKernel pres_kernel(int R) {
         }
     }
     return nullptr;
+}
+
+template <Form F>
+PresKernel pair_kernel(int R) {
+    switch (R) {
+        case 2: return k_res_pair<2, F>;
+        case 3: return k_res_pair<3, F>;
+        case 4: return k_res_pair<4, F>;
+        default: return nullptr;
+    }
 }
 
 using VelKernel = void (*)(const VelArgs);
@@ -980,9 +1236,12 @@ VelKernel vel_kernel(int R) {
 // shared: beside other cases' loops the product of a sweep's time and the
 // multiprocessors it holds counts instead, so that as many loops as possible
 // run at once.
-enum class Loop { kPres, kVel, kVelWide };
+enum class Loop { kPres, kVel, kVelWide, kPair };
 bool fits(const ResPlan& pl, Loop loop) {
     if (rim_of(pl) + 4 > NT) return false;
+    if (loop == Loop::kPair)
+        return (pl.bx + 2) * (pl.by + 2) <= NT && pair_plane_words(pl) <= kPairPlane &&
+               pair_halo(pl) <= kPairFetch * NT;
     if (loop == Loop::kVelWide)
         return pl.bx * pl.by <= NT && Edges(pl).words(pl.by) <= wide_plane(pl.bz) && kGroup * (rim_of(pl) + 4) <= NT;
     return inner0_of(pl) + inner_of(pl) <= NT && (pl.bx + kPad) * (pl.by + 2) <= plane_of(pl.bz) &&
@@ -1003,6 +1262,7 @@ ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], Loop loop = Loop
                 if (by < 2 || (P.ny + by - 1) / by != py) continue;
                 ResPlan pl;
                 pl.bx = bx; pl.by = by; pl.bz = R;
+                pl.pair = loop == Loop::kPair;
                 pl.px = px; pl.py = py; pl.pz = pz;
                 if (!fits(pl, loop)) continue;
                 const double halo = 2.0 * ((px > 1 ? by * R : 0) + (py > 1 ? bx * R : 0) + (pz > 1 ? bx * by : 0));
@@ -1031,6 +1291,7 @@ size_t vel_bytes(int R) {
     }
 }
 size_t packets(const ResPlan& p) {
+    if (p.pair) return (size_t)p.boxes() * p.bx * p.by * p.bz;
     return p.bz > 0 ? (size_t)p.boxes() * slots_of(p) : 0;
 }
 
@@ -1061,6 +1322,11 @@ int resident_setup(const Resident& r) {
         opt_in(pres_kernel<Form::kPasses, true>(r.pres.bz));
         opt_in(pres_kernel<Form::kOrdered, false>(r.pres.bz));
     }
+    if (r.pres2.bz > 0) {
+        opt_in(pair_kernel<Form::kPasses>(r.pres2.bz));
+        opt_in(pair_kernel<Form::kOrdered>(r.pres2.bz));
+        opt_in(pair_kernel<Form::kStretched>(r.pres2.bz));
+    }
     if (r.nupres.bz > 0) opt_in(pres_kernel<Form::kStretched, false>(r.nupres.bz));
     if (r.pres_shared.bz > 0) opt_in(pres_kernel<Form::kPasses, false>(r.pres_shared.bz));
     for (const ResPlan& p : {r.vel, r.vel_shared})
@@ -1071,6 +1337,8 @@ int resident_setup(const Resident& r) {
 void resident_plan(const Params& P, int sms, Resident* r) {
     r->pres = make_plan(P, sms, kPresR);
     r->nupres = make_plan(P, sms, kNuPresR);
+    r->pres2 = make_plan(P, sms, kPairR, Loop::kPair);
+    r->nupres2 = r->pres2;
     r->vel = make_plan(P, sms, kVelR, Loop::kVel);
     if (r->vel.bz == 0) r->vel = make_plan(P, sms, kVelWideR, Loop::kVelWide);
     r->pres_shared = make_plan(P, sms, kPresR, Loop::kPres, true);
@@ -1081,7 +1349,7 @@ void resident_alloc(Resident* r, cudaStream_t st) {
     // both parities of the pressure packets, then of the momentum packets
     // (apart: a momentum packet's words must not be read as pressure
     // packets), then the epoch words
-    const size_t np = 2 * std::max({packets(r->pres), packets(r->nupres), packets(r->pres_shared)}),
+    const size_t np = 2 * std::max({packets(r->pres), packets(r->nupres), packets(r->pres2), packets(r->pres_shared)}),
                  nv = 2 * std::max(packets(r->vel), packets(r->vel_shared));
     if (np + nv == 0 || r->work.pk) return;
     const size_t bytes = np * sizeof(unsigned long long) + nv * sizeof(Packet3) + 16 +
@@ -1120,7 +1388,7 @@ cudaError_t launch_pres(PresKernel k, const Params& P, cudaStream_t st, const Re
     a.half = packets(pl);
     a.ctl = w.ctl;
     a.status = status;
-    const cudaError_t e = launch_coop((const void*)k, pl.boxes(), pres_smem(pl.bz), st, &a);
+    const cudaError_t e = launch_coop((const void*)k, pl.boxes(), pl.pair ? pair_smem(pl) : pres_smem(pl.bz), st, &a);
     if (e == cudaSuccess) WF_COUNT_LAUNCH();
     else cudaGetLastError();
     return e;
@@ -1130,7 +1398,8 @@ cudaError_t launch_pres(PresKernel k, const Params& P, cudaStream_t st, const Re
 cudaError_t launch_res_pres(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w, const float* c3,
                             const float* ainv, const float* rhs, const float* pin, float* pout, float* pprev,
                             float* stack, int n, int* status, bool ordered) {
-    const PresKernel k = stack     ? pres_kernel<Form::kPasses, true>(pl.bz)
+    const PresKernel k = pl.pair   ? ordered ? pair_kernel<Form::kOrdered>(pl.bz) : pair_kernel<Form::kPasses>(pl.bz)
+                         : stack   ? pres_kernel<Form::kPasses, true>(pl.bz)
                          : ordered ? pres_kernel<Form::kOrdered, false>(pl.bz)
                                    : pres_kernel<Form::kPasses, false>(pl.bz);
     return launch_pres(k, P, st, pl, w, c3, ainv, rhs, pin, pout, pprev, stack, n, status);
@@ -1139,7 +1408,7 @@ cudaError_t launch_res_pres(const Params& P, cudaStream_t st, const ResPlan& pl,
 cudaError_t launch_res_nupres(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w,
                               const float* coef, const float* bp, const float* pin, float* pout, float* pprev, int n,
                               int* status) {
-    return launch_pres(pres_kernel<Form::kStretched, false>(pl.bz), P, st, pl, w, coef, coef + 6 * (size_t)P.N, bp, pin,
+    return launch_pres(pl.pair ? pair_kernel<Form::kStretched>(pl.bz) : pres_kernel<Form::kStretched, false>(pl.bz), P, st, pl, w, coef, coef + 6 * (size_t)P.N, bp, pin,
                        pout, pprev, nullptr, n, status);
 }
 

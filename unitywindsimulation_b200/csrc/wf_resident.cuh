@@ -12,6 +12,7 @@ namespace wf {
 // a thread owns (a z column); bz == 0: the grid does not fit on chip.
 struct ResPlan {
     int bx = 0, by = 0, bz = 0, px = 0, py = 0, pz = 0;
+    bool pair = false;   // pressure loop that runs two sweeps a halo trip
     int boxes() const { return px * py * pz; }
 };
 
@@ -28,9 +29,12 @@ struct ResWork {
 struct Resident {
     ResPlan pres;      // uniform pressure loops
     ResPlan nupres;    // non-uniform pressure loop
+    ResPlan pres2, nupres2;  // the same, two sweeps a halo trip, where that is faster
     ResPlan vel;       // momentum loop
     ResPlan pres_shared, vel_shared;  // the same beside other cases' loops: fewest multiprocessors
     ResWork work;
+    const ResPlan& pres_alone() const { return pres2.bz > 0 ? pres2 : pres; }
+    const ResPlan& nupres_alone() const { return nupres2.bz > 0 ? nupres2 : nupres; }
     bool ok(const ResPlan& p) const { return p.bz > 0 && work.pk != nullptr; }
 };
 

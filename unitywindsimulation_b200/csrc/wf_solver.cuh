@@ -137,7 +137,8 @@ inline bool loops_on_chip(const wf_solver* h, const ResPlan& p) { return h->resi
 // rule, 28800 with shared splits whatever their size (loops of more than half
 // the GPU each wait for it to empty).
 inline const ResPlan& pres_plan(const wf_solver* h) {
-    return h->in_batch && 2 * h->res.pres_shared.boxes() <= h->num_sms ? h->res.pres_shared : h->res.pres;
+    if (!h->in_batch) return h->res.pres_alone();
+    return 2 * h->res.pres_shared.boxes() <= h->num_sms ? h->res.pres_shared : h->res.pres;
 }
 inline const ResPlan& vel_plan(const wf_solver* h) {
     static const ResPlan none;
