@@ -86,6 +86,14 @@ def test_stretched_mesh_bit_identical(built, kw):
     assert np.array_equal(a.get_face_flux(), b.get_face_flux())
 
 
+# the adjoint's momentum iterates, forward and transposed, in the other splits (4
+# to 15 cells a thread)
+@pytest.mark.parametrize("grid", [(72, 40, 72), (88, 41, 77), (100, 50, 75), (103, 53, 104), (128, 64, 96), (130, 61, 110),
+                                  (149, 61, 103)], ids=lambda g: "%dx%dx%d" % g)
+def test_adjoint_momentum_iterates(built, grid):
+    test_adjoint_iterates(built, grid)
+
+
 @pytest.mark.parametrize("grid", [(24, 12, 16), (41, 21, 30)], ids=lambda g: "%dx%dx%d" % g)
 def test_adjoint_iterates(built, grid):
     """Recorded forward step bit for bit; the reversed step to the rounding

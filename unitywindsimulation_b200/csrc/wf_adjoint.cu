@@ -923,6 +923,17 @@ int adj_check_waits(wf_adjoint* a) {
 
 // On-chip pressure loops, or nullptr where the solver runs the pass kernels.
 const wf::Resident* adj_resident(const wf_adjoint* a) { return a->h->resident && a->h->dstat ? &a->res : nullptr; }
+// n momentum sweeps from u^0 on chip with every iterate kept (u^k at u0 + k step);
+// the transposed sweeps are the forward ones with A^T and no right-hand side.  One
+// sweep a launch moves all 82 bytes of a cell: 8.2 us on 128 x 64 x 96; on chip only
+// the iterate leaves: 7.5 (4.7 without it).  False: not run, the caller launches its
+// sweeps.
+bool vel_on_chip(wf_adjoint* a, const float* A, const float* iD, const float* b, float* u0, int n, long long step) {
+    const wf::Resident* r = adj_resident(a);
+    return r && n >= 2 && r->ok(r->vel) &&
+           wf::launch_res_vel(a->h->P, a->st, r->vel, r->work, A, iD, b, u0, nullptr, nullptr, n, a->h->dstat, u0,
+                              step) == cudaSuccess;
+}
 
 float* V(const wf_adjoint* a, float* base, int k) { return base + (size_t)k * 3 * a->N; }
 float* S(const wf_adjoint* a, float* base, int k) { return base + (size_t)k * a->N; }
@@ -996,8 +1007,9 @@ int record_step(wf_adjoint* a, Tape& t, const float* u_in, const float* p_in, in
     wf::launch_vel_precompute(P, h->B, st, h->fl, t.uT, t.p0, h->eddy, h->face, nullptr, h->drag, t.D, t.b);
     wf::launch_vel_coef_ptr(P, st, h->fl, t.uT, h->eddy, h->face, t.D, t.A, t.iD);
     WFA_CUDA(cudaMemcpyAsync(V(a, t.uit, 0), t.uT, v, cudaMemcpyDeviceToDevice, st));
-    for (int k = 0; k < a->nV; ++k)
-        wf::launch_vel_sweep1_ptr(P, st, t.A, t.iD, t.b, V(a, t.uit, k), V(a, t.uit, k + 1));
+    if (!vel_on_chip(a, t.A, t.iD, t.b, t.uit, a->nV, 3 * (long long)N))
+        for (int k = 0; k < a->nV; ++k)
+            wf::launch_vel_sweep1_ptr(P, st, t.A, t.iD, t.b, V(a, t.uit, k), V(a, t.uit, k + 1));
     const float* ustar = V(a, t.uit, a->nV);
     WFA_CUDA(cudaMemcpyAsync(t.uout, ustar, v, cudaMemcpyDeviceToDevice, st));
     WFA_CUDA(cudaMemcpyAsync(t.pout, t.p0, s, cudaMemcpyDeviceToDevice, st));
@@ -1106,7 +1118,8 @@ int adjoint_step(wf_adjoint* a, const Tape& t, int phases) {
                                                                            V(a, a->Wv, n));
         const bool v4 = n > 1 && wf::quad_ok(P, {a->AT, t.iD, V(a, a->Wv, n), V(a, a->Wv, n - 1)});
         const dim3 b4 = wf::groups_block(P), g4 = wf::grid_for(P.nx / 4, P.ny, P.nz, b4);
-        for (int k = n - 1; k >= 1; --k) {
+        const bool chip = vel_on_chip(a, a->AT, t.iD, nullptr, V(a, a->Wv, n), n - 1, -3 * (long long)N);
+        for (int k = n - 1; k >= 1 && !chip; --k) {
             if (v4)
                 wf::k_adj_vsweepT4<<<g4, b4, 0, st>>>(P, a->AT, t.iD, V(a, a->Wv, k + 1), V(a, a->Wv, k));
             else
@@ -1184,6 +1197,7 @@ int wf_adj_create(wf_solver* h, wf_adjoint** out) {
     if (ok) ok = ensure_tapes(a, 1) == WF_OK;
     if (ok) {
         a->res.pres = h->res.pres;
+        a->res.vel = h->res.vel;
         wf::resident_alloc(&a->res, a->st);
     }
     if (ok) ok = cudaStreamSynchronize(a->st) == cudaSuccess;

@@ -743,6 +743,8 @@ struct VelArgs {
     unsigned* ctl;
     int* status;
     float* stream;   // k_res_vel_wide: the words read in every sweep
+    float* stack;    // iterate k of every cell goes to stack + k step
+    long long step;
 };
 
 // receive() for three components, CS floats apart in the shared box.  Every
@@ -791,7 +793,9 @@ __device__ __forceinline__ bool receive3(const Links& l, float* v, const Packet3
     return true;
 }
 
-template <int R>
+// STACK: every iterate of every cell goes to a.stack (non-fluid cells keep the
+// input's value); bv nullptr: 0.
+template <int R, bool STACK>
 __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelArgs a) {
     extern __shared__ __align__(16) float sm[];
     constexpr bool kShared = R > kVelRegR;
@@ -843,7 +847,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
         const bool fluid = d0[r] != 0.f;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const float v = fluid ? __ldg(a.bv + c * N + i) : 0.f;
+            const float v = fluid && a.bv ? __ldg(a.bv + c * N + i) : 0.f;
             if (kShared) priv[(c * R + r) * NT + tid] = v;
             else bb[kShared ? 0 : c][kShared ? 0 : r] = v;
             if (c > 0) {
@@ -899,6 +903,18 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
                 for (int c = 0; c < 3; ++c) out[c * N + i0 + r * sxy] = u[c][r];
             }
     };
+    auto keep = [&](int k) {
+        float* s = a.stack + k * a.step;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (inxy && b.z0 + r < a.nz) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const size_t i = c * N + i0 + r * sxy;
+                    s[i] = d0[r] != 0.f ? u[c][r] : __ldg(a.uin + i);
+                }
+            }
+    };
     __syncthreads();
     Packet3 *pk = a.pk, *pk_next = a.pk + a.half;
     unsigned ep = base;
@@ -921,6 +937,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
 #pragma unroll
                 for (int r = 0; r < R; ++r) cur[c * CS + r * PS] = u[c][r];
         }
+        if (STACK) keep(k);
         if (gridDim.x > 1) bad = !receive3<fetch_max(R), CS>(l, sm, pk, ep, hu, hd);
         if (__syncthreads_or(bad)) break;
         Packet3* t = pk;
@@ -934,7 +951,8 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
         if (a.uprev) emit(a.uprev);
         ends();
         middle();
-        emit(a.uout);
+        if (STACK) keep(a.n);
+        if (a.uout) emit(a.uout);
     }
     epoch_end(a.ctl, base, (unsigned)a.n + 1u);
 }
@@ -998,7 +1016,7 @@ __device__ __forceinline__ float ld_stream(const float* p) {
     return v;
 }
 
-template <int R>
+template <int R, bool STACK>
 __global__ void __launch_bounds__(NT, 1) k_res_vel_wide(const __grid_constant__ VelArgs a) {
     extern __shared__ __align__(16) float sm[];
     constexpr int PS = Wide<R>::PS, CS = R * PS, BUF = 3 * CS;      // plane, component, box
@@ -1080,7 +1098,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel_wide(const __grid_constant__ 
 #pragma unroll
         for (int w = 0; w < 6; ++w) {
             const float* src = w == 0 ? a.iD : w < 4 ? a.bv + (w - 1) * N : a.iD + (w - 3) * N;
-            const float v = w == 0 ? d0 : fluid ? __ldg(src + i) : 0.f;
+            const float v = w == 0 ? d0 : fluid && (a.bv || w > 3) ? __ldg(src + i) : 0.f;
             if (w < NR) wr[w < NR ? w : 0][r] = v;
             else if (w < NR + NS) priv[((w - NR) * R + r) * NT + tid] = v;
             else str[(r * S + w - NR - NS) * NT] = v;
@@ -1127,6 +1145,15 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel_wide(const __grid_constant__ 
             plane(r, bel, v, w[0]);
         }
     };
+    auto keep = [&](int k, int r, const float* v, float d0) {
+        if (!inxy || b.z0 + r >= a.nz) return;
+        float* s = a.stack + k * a.step;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const size_t i = c * N + i0 + r * sxy;
+            s[i] = d0 != 0.f ? v[c] : __ldg(a.uin + i);
+        }
+    };
     __syncthreads();
     fetch(R - 1);
     Packet3 *pk = a.pk, *pk_next = a.pk + a.half;
@@ -1137,7 +1164,8 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel_wide(const __grid_constant__ 
         ++ep;
         const float* cu = sm + at;
         float* nb = sm + (BUF - at);
-        sweep(cu, [&](int r, const float*, const float* v, float) {
+        sweep(cu, [&](int r, const float*, const float* v, float d0) {
+            if (STACK) keep(k, r, v, d0);
             if (own) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) nb[o0 + c * CS + r * PS] = v[c];
@@ -1159,7 +1187,8 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel_wide(const __grid_constant__ 
         if (tid == 0 && a.status) atomicExch(a.status, 1);
     } else {
         sweep(sm + at, [&](int r, const float* old, const float* v, float d0) {
-            if (inxy && b.z0 + r < a.nz && d0 != 0.f) {
+            if (STACK) keep(a.n, r, v, d0);
+            if (a.uout && inxy && b.z0 + r < a.nz && d0 != 0.f) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     a.uout[c * N + i0 + r * sxy] = v[c];
@@ -1212,17 +1241,18 @@ PresKernel pair_kernel(int R) {
 }
 
 using VelKernel = void (*)(const VelArgs);
+template <bool STACK>
 VelKernel vel_kernel(int R) {
     switch (R) {
-        case 2: return k_res_vel<2>;
-        case 3: return k_res_vel<3>;
-        case 4: return k_res_vel<4>;
-        case 6: return k_res_vel<6>;
-        case 8: return k_res_vel<8>;
-        case 10: return k_res_vel_wide<10>;
-        case 12: return k_res_vel_wide<12>;
-        case 14: return k_res_vel_wide<14>;
-        case 15: return k_res_vel_wide<15>;
+        case 2: return k_res_vel<2, STACK>;
+        case 3: return k_res_vel<3, STACK>;
+        case 4: return k_res_vel<4, STACK>;
+        case 6: return k_res_vel<6, STACK>;
+        case 8: return k_res_vel<8, STACK>;
+        case 10: return k_res_vel_wide<10, STACK>;
+        case 12: return k_res_vel_wide<12, STACK>;
+        case 14: return k_res_vel_wide<14, STACK>;
+        case 15: return k_res_vel_wide<15, STACK>;
         default: return nullptr;
     }
 }
@@ -1329,8 +1359,9 @@ int resident_setup(const Resident& r) {
     }
     if (r.nupres.bz > 0) opt_in(pres_kernel<Form::kStretched, false>(r.nupres.bz));
     if (r.pres_shared.bz > 0) opt_in(pres_kernel<Form::kPasses, false>(r.pres_shared.bz));
+    if (r.vel.bz > 0) opt_in(vel_kernel<true>(r.vel.bz));
     for (const ResPlan& p : {r.vel, r.vel_shared})
-        if (p.bz > 0) opt_in(vel_kernel(p.bz));
+        if (p.bz > 0) opt_in(vel_kernel<false>(p.bz));
     return e == cudaSuccess ? WF_OK : WF_ERR_CUDA;
 }
 
@@ -1414,7 +1445,7 @@ cudaError_t launch_res_nupres(const Params& P, cudaStream_t st, const ResPlan& p
 
 cudaError_t launch_res_vel(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w, const float* A,
                            const float* iD, const float* bv, const float* uin, float* uout, float* uprev, int n,
-                           int* status) {
+                           int* status, float* stack, long long step) {
     VelArgs a = {};
     a.nx = P.nx; a.ny = P.ny; a.nz = P.nz; a.n = n;
     a.pl = pl;
@@ -1425,7 +1456,10 @@ cudaError_t launch_res_vel(const Params& P, cudaStream_t st, const ResPlan& pl, 
     a.ctl = w.ctl;
     a.status = status;
     a.stream = w.stream;
-    const cudaError_t e = launch_coop((const void*)vel_kernel(pl.bz), pl.boxes(), vel_bytes(pl.bz), st, &a);
+    a.stack = stack;
+    a.step = step;
+    const VelKernel k = stack ? vel_kernel<true>(pl.bz) : vel_kernel<false>(pl.bz);
+    const cudaError_t e = launch_coop((const void*)k, pl.boxes(), vel_bytes(pl.bz), st, &a);
     if (e == cudaSuccess) WF_COUNT_LAUNCH();
     else cudaGetLastError();
     return e;

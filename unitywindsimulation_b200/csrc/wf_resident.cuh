@@ -67,9 +67,11 @@ cudaError_t launch_res_nupres(const Params& P, cudaStream_t st, const ResPlan& p
 // n >= 2 momentum sweeps u = (1/D) (sum_f A_f u_f + b) from uin in one
 // launch: A holds A_E..A_D, iD the three components of 1/D.  The iterates of
 // k_vel_sweep4 bit for bit; uout (uprev, nullable) receives iterate n (n - 1)
-// on fluid cells and may not alias uin.
+// on fluid cells and may not alias uin.  stack (nullable; uout may then be
+// nullptr): every iterate k = 1..n of every cell at stack + k step, non-fluid cells
+// with uin's value.  bv nullptr: 0.
 cudaError_t launch_res_vel(const Params& P, cudaStream_t st, const ResPlan& pl, const ResWork& w, const float* A,
                            const float* iD, const float* bv, const float* uin, float* uout, float* uprev, int n,
-                           int* status);
+                           int* status, float* stack = nullptr, long long step = 0);
 
 }  // namespace wf
