@@ -20,14 +20,15 @@
 //
 // What bounds it: the trip of the packets (470 cycles within a die, 900 across,
 // measured SM to SM) and the instructions of a column, one warp after another;
-// not memory.  Measured, us a sweep: 1.1 on 64 x 32 x 48, 1.13 on 80 x 40 x 40,
-// 1.75 on 100 x 50 x 100, 2.3 on 128 x 64 x 96, 3.5 on 149 x 61 x 103.  Whole
-// steps, with the four-sweep passes before: 623 -> 310 us (64 x 32 x 48, PISO,
-// 90 pressure sweeps), 5077 -> 1467 us (80 x 40 x 40, 1000), 2425 -> 1059 us (100 x 50 x
-// 100, 400), 1278 -> 1027 us (128 x 64 x 96, 90), 1396 -> 1186 us (149 x 61 x 103, 90),
-// 9761 -> 8258 us (100 x 50 x 100 stretched mesh, 2000).  With the momentum loop
-// on chip too: 310 -> 269 us (64 x 32 x 48, 50 sweeps), 1467 -> 1399 us (80 x 40 x 40,
-// 100), 1059 -> 982 us (100 x 50 x 100, 50), 8258 -> 6753 us (stretched mesh, 800).
+// not memory.  Measured, us a pressure sweep: 0.77 on 64 x 32 x 48 and 0.81 on 80 x
+// 40 x 40 (two sweeps a trip, k_res_pair; 1.10 and 1.16 with one), 1.74 on 100 x 50 x
+// 100, 2.3 on 128 x 64 x 96, 3.5 on 149 x 61 x 103; a momentum sweep: 1.30, 1.41,
+// 2.96, 4.7 and 6.6.  Whole steps, with one launch for every one to four sweeps
+// before: 623 -> 237 us (64 x 32 x 48, PISO, 50 momentum and 90 pressure sweeps),
+// 5077 -> 1026 us (80 x 40 x 40, 100 and 1000), 2429 -> 947 us (100 x 50 x 100, 50 and
+// 400), 1279 -> 977 us (128 x 64 x 96, 50 and 90, its fields read back), 1397 -> 975 us
+// (149 x 61 x 103, 50 and 90), 9759 -> 6226 us (100 x 50 x 100 stretched mesh, 800 and
+// 2000).
 //
 // The launch is cooperative, so all blocks are resident and every packet
 // that is waited for will be sent.  The waits are bounded all the same
@@ -969,7 +970,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
 // What bounds it: the shared-memory reads (five a cell and component) and the
 // streamed words while it computes, then a halo trip of 33 KB a box.  Measured,
 // us a sweep: 4.7 on 128 x 64 x 96 (3.1 without the exchange, 4.1 without the
-// streamed words), 6.7 on 149 x 61 x 103, against 5.6 and 11 for one sweep a
+// streamed words), 6.6 on 149 x 61 x 103, against 6.1 and 11.6 for one sweep a
 // launch, which moves all 82 bytes of a cell through L2.  Halo cells fetched
 // while the planes are computed, with or without waiting, cost 0.2 us for each
 // packet of a thread; all at the end is the fastest.  E and W halo columns
