@@ -34,3 +34,18 @@ def test_blocks_by_extents(built, grid, block):
         assert np.array_equal(a.get_field(f), b.get_field(f)), _lib.FIELD_NAMES[f]
     for f in (_lib.FIELD_VEL_LAST_TIME, _lib.FIELD_PRES):
         assert rel_l2(a.get_field(f), o.get_field(f)) <= REL_TOL, _lib.FIELD_NAMES[f]
+
+
+@pytest.mark.parametrize("nx", [24, 27])
+def test_step_equals_its_operations(built, nx):
+    """Inside a step the pre-computes also store the sweeps' reciprocals; the
+    operations one by one compute them apart."""
+    case = cases.small_case(nx=nx, piso=False, les=False)
+    a, b = FvmSolverCuda(case.cfg), FvmSolverCuda(case.cfg)
+    for s in (a, b):
+        cases.apply_case(s, case)
+    a.Step(1)
+    b.op("vel_precompute"); b.op("vel_sweeps", case.cfg.vel_iters); b.op("pres_precompute")
+    b.op("pres_sweeps", case.cfg.pres_iters); b.op("apply_pres"); b.op("apply_vel"); b.op("end_step")
+    f = _lib.FIELD_VEL_LAST_TIME
+    assert np.array_equal(a.get_field(f), b.get_field(f))

@@ -269,9 +269,11 @@ int do_pres_precompute(wf_solver* h) {
     // the fast path's pressure face coefficients come out of the same pass
     // (they depend on D only, like the cache generation they are keyed by)
     float* c3 = h->fast ? h->pcoef : nullptr;
-    wf::launch_pres_precompute(h->P, h->B, h->st, h->fl, h->vb[h->iF], h->pr, h->Dv, cur_inv_d(h), h->Dp, h->bp, c3);
+    wf::launch_pres_precompute(h->P, h->B, h->st, h->fl, h->vb[h->iF], h->pr, h->Dv, cur_inv_d(h), h->Dp, h->bp, c3,
+                               h->in_step && c3 ? c3 + 3 * (size_t)h->P.N : nullptr);
     WF_CHECK_LAUNCH();
     if (c3) h->c3_gen = h->d_gen;
+    h->ainv_step = h->in_step && c3;  // nothing between here and the sweeps changes Dp
     return WF_OK;
 }
 
@@ -402,6 +404,7 @@ int enqueue_step(wf_solver* h) {
     const int s = enqueue_step_body(h);
     h->in_step = false;
     h->vcoef_step = false;
+    h->ainv_step = false;
     return s;
 }
 
@@ -1038,6 +1041,7 @@ int wf_step_phases(wf_solver* h, float* phase_ms) {
     } while (false);
     h->in_step = false;
     h->vcoef_step = false;
+    h->ainv_step = false;
     if (phase >= 0 && phase < WF_PHASE_COUNT) nvtxRangePop();
     h->launches += wf::g_launches - l0;
     if (st != WF_OK) return st;

@@ -584,10 +584,12 @@ __global__ void k_vel_sweep(const __grid_constant__ Params P, const float* __res
 // c3 (nullable): also stores the pressure sweeps' face coefficients c_E,
 // c_N, c_U (three planes; (dv/den) DInv / dx on fluid-fluid faces, else 0),
 // the values k_pres_coef computes from the same D, as the same products.
+// ainv (nullable): also stores 1/Dp, 0 on non-fluid cells (launch_inv's values).
 __global__ void k_pres_precompute(const __grid_constant__ Params P, const Bnd B, const uint8_t* __restrict__ fl,
                                   const float* __restrict__ u, const float* __restrict__ pr,
                                   const float* __restrict__ Dv, const float* __restrict__ iD,
-                                  float* __restrict__ Dp, float* __restrict__ bp, float* __restrict__ c3) {
+                                  float* __restrict__ Dp, float* __restrict__ bp, float* __restrict__ c3,
+                                  float* __restrict__ ainv) {
     Cell c;
     if (!cell_of_thread(P, c)) return;
     (void)fl;
@@ -622,6 +624,7 @@ __global__ void k_pres_precompute(const __grid_constant__ Params P, const Bnd B,
 #pragma unroll
             for (int a = 0; a < 3; ++a) c3[a * N + c.i] = 0.f;
         }
+        if (ainv) ainv[c.i] = 0.f;
         return;
     }
     float DP = 0.f, bP = 0.f;
@@ -669,6 +672,7 @@ __global__ void k_pres_precompute(const __grid_constant__ Params P, const Bnd B,
     }
     Dp[c.i] = DP;
     bp[c.i] = bP;
+    if (ainv) ainv[c.i] = 1.f / DP;
 }
 
 // CSPresCorrectRhieChow, FvmColl.compute:2790-2848.  pin == nullptr reads as
@@ -1155,8 +1159,9 @@ void launch_vel_sweep(const Params& P, cudaStream_t st, const float* uI, const f
     WF_LAUNCH(k_vel_sweep, uI, uT, eddy, Dv, iD, bv, uo);
 }
 void launch_pres_precompute(const Params& P, const Bnd& B, cudaStream_t st, const uint8_t* fl, const float* u,
-                            const float* pr, const float* Dv, const float* iD, float* Dp, float* bp, float* c3) {
-    WF_LAUNCH(k_pres_precompute, B, fl, u, pr, Dv, iD, Dp, bp, c3);
+                            const float* pr, const float* Dv, const float* iD, float* Dp, float* bp, float* c3,
+                            float* ainv) {
+    WF_LAUNCH(k_pres_precompute, B, fl, u, pr, Dv, iD, Dp, bp, c3, ainv);
 }
 void launch_pres_sweep(const Params& P, cudaStream_t st, const float* pin, const float* Dv, const float* iD,
                        const float* Dp, const float* bp, float* pout) {

@@ -29,7 +29,8 @@ void launch_vel_sweep(const Params& P, cudaStream_t st, const float* uI, const f
 // iD (nullable): cached 1/D of the same D (bit-identical to dividing).
 void launch_pres_precompute(const Params& P, const Bnd& B, cudaStream_t st, const uint8_t* fl, const float* u,
                             const float* pr, const float* Dv, const float* iD, float* Dp, float* bp,
-                            float* c3 = nullptr);
+                            float* c3 = nullptr,
+                            float* ainv = nullptr);
 void launch_pres_sweep(const Params& P, cudaStream_t st, const float* pin, const float* Dv, const float* iD,
                        const float* Dp, const float* bp, float* pout);
 void launch_apply_pres(const Params& P, cudaStream_t st, const uint8_t* fl, const float* pc, float* pr);

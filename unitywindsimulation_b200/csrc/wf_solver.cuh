@@ -67,6 +67,7 @@ struct wf_solver {
     // the momentum pre-compute of the step in progress wrote vcoef (A and
     // 1/D) for the current D; the step's sweeps take them as they are
     bool vcoef_step = false;
+    bool ainv_step = false;   // the same for 1/Dp (pcoef + 3N) and the pressure pre-compute
     // scratch
     double* part = nullptr;
     double* dsum = nullptr;   // 4 doubles

@@ -795,6 +795,10 @@ const float* pres_coef(wf_solver* h, bool piso) {
         k_pres_coef<<<cells_grid(P), cells_block(P), 0, h->st>>>(P, h->fl, h->Dv, iDc, c3);
         h->c3_gen = h->d_gen;
     }
+    if (!piso && h->in_step && h->ainv_step) {  // this step's pressure pre-compute stored it
+        h->ainv_step = false;
+        return rhs;
+    }
     WF_COUNT_LAUNCH();
     if (piso) {
         k_piso_pre<<<cells_grid(P), cells_block(P), 0, h->st>>>(P, h->fl, h->Dv, iDc, h->aodu, ainv, rhs);
