@@ -289,7 +289,7 @@ struct PresArgs {
     int nx, ny, nz, n;
     ResPlan pl;
     const float *c, *ainv, *rhs;   // c: c_E, c_N, c_U planes, or the six face planes
-    const uint8_t* nbm;            // neighbour masks (non-uniform)
+    const uint8_t* nbm;            // neighbour masks; bit 6: fluid
     const float* pin;
     float *pout, *pprev, *stack;
     unsigned long long* pk;
@@ -297,6 +297,41 @@ struct PresArgs {
     unsigned* ctl;
     int* status;
 };
+
+// The loops read every neighbour, fluid or not, through a coefficient that is 0 on
+// faces of non-fluid cells.  0 times an infinity or a NaN is NaN, and a fluid cell
+// without fluid neighbours has 1/Dp = inf and the value NaN; so a cell whose 1/D is 0
+// (not fluid, or beyond the domain) is 0 by selection, not by the product, and no NaN
+// crosses a wall (the kernels of one sweep a launch skip non-fluid neighbours by the
+// mask).  Up to kRegR cells a thread the column's cells to clear are bits of a word, and
+// a warp without any skips them all (100 x 50 x 100, 400 sweeps: step 920 us, 942 with a
+// select at every cell); above, the word costs spills (128 x 64 x 96 with its copies:
+// 1092 us against 984) and every cell selects.  The pair kernel does not store such a
+// cell and drops its packet: it stays 0.
+template <int First, int Last, int M>
+__device__ __forceinline__ void clear_walls(unsigned walls, float (&v)[M]) {
+#pragma unroll
+    for (int r = First; r <= Last; ++r)
+        if (walls >> r & 1u) v[r] = 0.f;
+}
+template <bool kSelect>
+__device__ __forceinline__ float scaled(float inv, float sum) {
+    return !kSelect || inv != 0.f ? inv * sum : 0.f;
+}
+__device__ __forceinline__ bool fluid_bit(const PresArgs& a, int i) { return (__ldg(a.nbm + i) & 64u) != 0; }
+// Cell i of the input iterate; where the mask decides, what a buffer holds on
+// non-fluid cells is no iterate.
+template <Form F>
+__device__ __forceinline__ float input_of(const PresArgs& a, int i) {
+    const float v = __ldg(a.pin + i);
+    return F == Form::kPasses || fluid_bit(a, i) ? v : 0.f;
+}
+// Whether cell i of the result is stored: as in the kernel whose sums F are, those of
+// the passes by 1/Dp, the others by the mask.
+template <Form F>
+__device__ __forceinline__ bool written(const PresArgs& a, int i, float inv) {
+    return F == Form::kPasses ? inv != 0.f : fluid_bit(a, i);
+}
 
 // Above kRegR cells a thread 1/Dp and the right-hand side live in shared
 // memory instead of registers.
@@ -338,25 +373,28 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
     if (a.pin) {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            if (inxy && b.z0 + r < a.nz) p[r] = __ldg(a.pin + i0 + r * sxy);
+            if (inxy && b.z0 + r < a.nz) p[r] = input_of<F>(a, i0 + r * sxy);
             if (own) sm[r * PS + o0] = p[r];
         }
-        if (inxy && b.z0 > 0) hd = __ldg(a.pin + i0 - sxy);
-        if (inxy && b.z0 + R < a.nz) hu = __ldg(a.pin + i0 + R * sxy);
+        if (inxy && b.z0 > 0) hd = input_of<F>(a, i0 - sxy);
+        if (inxy && b.z0 + R < a.nz) hu = input_of<F>(a, i0 + R * sxy);
         if (tid < b.rim + 4) {  // the threads that fetch from plane 0 on
             const int hy = b.y0 + l.he / b.sx - 1, hx = b.x0 + l.he % b.sx - 1;
-            if (hx >= 0 && hx < a.nx && hy >= 0 && hy < a.ny)
-                for (int r = 0; r < R && b.z0 + r < a.nz; ++r)
-                    sm[r * PS + l.he] = __ldg(a.pin + (size_t)(b.z0 + r) * sxy + hy * a.nx + hx);
+            if (hx >= 0 && hx < a.nx && hy >= 0 && hy < a.ny) {
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    if (b.z0 + r < a.nz) sm[r * PS + l.he] = input_of<F>(a, (b.z0 + r) * sxy + hy * a.nx + hx);
+            }
         }
     }
     // the column's coefficients
     float cE[R], cW[R], cN[R], cS[R], cU[R], cD[NU ? R : 1], ai[kShared ? 1 : R], rh[kShared ? 1 : R];
+    unsigned walls = 0;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int i = i0 + r * sxy;
         bool in = inxy && b.z0 + r < a.nz;
-        if (NU && in) in = (__ldg(a.nbm + i) & 64u) != 0;  // solid cells hold no coefficients
+        if (NU && in) in = fluid_bit(a, i);  // solid cells hold no coefficients
         if (NU) {
             cE[r] = in ? __ldg(a.c + i) : 0.f;
             cW[r] = in ? __ldg(a.c + N + i) : 0.f;
@@ -373,6 +411,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
             if (r == 0) cD[0] = in && b.z0 > 0 ? __ldg(a.c + 2 * N + i - sxy) : 0.f;
         }
         const float e_ai = in ? __ldg(a.ainv + i) : 0.f;
+        if (!kShared && own && e_ai == 0.f) walls |= 1u << r;
         const float e_rh = in && a.rhs ? __ldg(a.rhs + i) : 0.f;
         if (kShared) {
             sai[r * NT + tid] = e_ai;
@@ -397,7 +436,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
         acc -= cS[r] * qs[r * PS];
         acc -= cU[r] * up;
         acc -= (NU ? cD[NU ? r : 0] : (r > 0 ? cU[r > 0 ? r - 1 : 0] : cD[0])) * below;
-        return inv_of(r) * (acc + (kShared ? sai[(R + r) * NT + tid] : rh[kShared ? 0 : r]));
+        return scaled<kShared>(inv_of(r), acc + (kShared ? sai[(R + r) * NT + tid] : rh[kShared ? 0 : r]));
     };
     // one sweep of the column from the iterate at `cur`; the two end cells come
     // first, so that their packets can leave before the rest is computed
@@ -413,10 +452,15 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
     unsigned ep = base;
     bool bad = false;
     const bool has_halo = gridDim.x > 1 && (tid & ~31) < b.inner0 + inner_of(a.pl);
+    const bool any_walls = !kShared && __any_sync(0xffffffffu, walls != 0);
     float v0, vT;
     auto ends = [&]() {
         v0 = cell(cur, 0, R > 1 ? p[R > 1 ? 1 : 0] : hu, hd);
         vT = R > 1 ? cell(cur, R - 1, hu, p[R > 1 ? R - 2 : 0]) : v0;
+        if (any_walls) {
+            if (walls & 1u) v0 = 0.f;
+            if (walls >> (R - 1) & 1u) vT = 0.f;
+        }
     };
     auto middle = [&]() {
         float below = p[0];
@@ -427,6 +471,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
             p[r] = cell(cur, r, r + 1 < R - 1 ? p[r + 1 < R ? r + 1 : 0] : top, below);
             below = old;
         }
+        if (any_walls) clear_walls<1, R - 2>(walls, p);
         p[0] = v0;
         p[R - 1] = vT;
     };
@@ -464,7 +509,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
         if (a.pprev) {
 #pragma unroll
             for (int r = 0; r < R; ++r)
-                if (inxy && b.z0 + r < a.nz && inv_of(r) != 0.f) a.pprev[i0 + r * sxy] = p[r];
+                if (inxy && b.z0 + r < a.nz && written<F>(a, i0 + r * sxy, inv_of(r))) a.pprev[i0 + r * sxy] = p[r];
         }
         ends();
         middle();
@@ -472,7 +517,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
         if (a.pout) {
 #pragma unroll
             for (int r = 0; r < R; ++r)
-                if (inxy && b.z0 + r < a.nz && inv_of(r) != 0.f) a.pout[i0 + r * sxy] = p[r];
+                if (inxy && b.z0 + r < a.nz && written<F>(a, i0 + r * sxy, inv_of(r))) a.pout[i0 + r * sxy] = p[r];
         }
     }
     epoch_end(a.ctl, base, (unsigned)a.n + 1u);
@@ -575,9 +620,14 @@ __global__ void __launch_bounds__(NT, 1) k_res_pair(const __grid_constant__ Pres
         const int row = lx == -2 ? w * (by + 4) + ly : lx == bx + 1 ? w * (by + 4) + by + ly : (ly + 2) * w + lx + 1;
         int2 t = make_int2(-1, (lz + 2) * PS + row);
         if (x >= 0 && x < a.nx && y >= 0 && y < a.ny && z >= 0 && z < a.nz) {
+            // a non-fluid cell stays 0: its packet is waited for like any other (the
+            // protocol needs both directions of a pair of boxes) and goes to the plane's
+            // corner word, which no column reads
+            const bool fluid = fluid_bit(a, (z * a.ny + y) * a.nx + x);
+            if (!fluid) t.y = (lz + 2) * PS;
             const int ox = lx < 0 ? -1 : lx >= bx, oy = ly < 0 ? -1 : ly >= by, oz = lz < 0 ? -1 : lz >= R;
             t.x = (id + ox + px * (oy + py * oz)) * cells + (lx - ox * bx) + bx * ((ly - oy * by) + by * (lz - oz * R));
-            if (a.pin) s0[t.y] = __ldg(a.pin + ((size_t)z * a.ny + y) * a.nx + x);
+            if (a.pin && fluid) s0[t.y] = __ldg(a.pin + (z * a.ny + y) * a.nx + x);
         }
         tab[e] = t;
     }
@@ -593,14 +643,14 @@ __global__ void __launch_bounds__(NT, 1) k_res_pair(const __grid_constant__ Pres
     const bool mine = own && col, lo = mine && z0 > 0, hi = mine && z0 + R < a.nz;
     // coefficients of the column's cells, j = 0 .. R + 1 for z = -1 .. R
     float cE[E], cW[E], cN[E], cS[E], cU[E], cD[NU ? E : 1], ai[E], rh[E];
+    unsigned keep = 0;   // cells that are stored; the others stay 0
 #pragma unroll
     for (int j = 0; j < E; ++j) {
         const int z = z0 + j - 1;
         const bool inz = col && z >= 0 && z < a.nz;
         bool in = inz && (own || (j > 0 && j <= R));
         const int i = inz ? z * sxy + i0 : 0;
-        if (mine && a.pin && j > 0 && j <= R && inz) s0[o + (j + 1) * PS] = __ldg(a.pin + i);
-        if (NU && in) in = (__ldg(a.nbm + i) & 64u) != 0;  // solid cells hold no coefficients
+        if (NU && in) in = fluid_bit(a, i);  // solid cells hold no coefficients
         if (NU) {
             cE[j] = in ? __ldg(a.c + i) : 0.f;
             cW[j] = in ? __ldg(a.c + N + i) : 0.f;
@@ -617,6 +667,8 @@ __global__ void __launch_bounds__(NT, 1) k_res_pair(const __grid_constant__ Pres
             if (j == 0) cD[0] = in && z > 0 ? __ldg(a.c + 2 * N + i - sxy) : 0.f;
         }
         ai[j] = in ? __ldg(a.ainv + i) : 0.f;
+        if ((j == 0 ? lo : j == R + 1 ? hi : col) && ai[j] != 0.f) keep |= 1u << j;
+        if (mine && a.pin && j > 0 && j <= R && ai[j] != 0.f) s0[o + (j + 1) * PS] = __ldg(a.pin + i);
         rh[j] = in && a.rhs ? __ldg(a.rhs + i) : 0.f;
     }
     // cell j of the column from the iterate at s
@@ -648,7 +700,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_pair(const __grid_constant__ Pres
         sweep(s0, 0, R + 1);
 #pragma unroll
         for (int j = 0; j < E; ++j)
-            if (j == 0 ? lo : j == R + 1 ? hi : col) s1[o + (j + 1) * PS] = v[j];
+            if (keep >> j & 1u) s1[o + (j + 1) * PS] = v[j];
     };
     __syncthreads();
     unsigned long long *pk = a.pk, *pk_next = a.pk + a.half;
@@ -666,7 +718,8 @@ __global__ void __launch_bounds__(NT, 1) k_res_pair(const __grid_constant__ Pres
             for (int j = 1; j <= R; ++j)
                 if (H > 0 && (R <= 4 || edge || j <= 2 || j >= R - 1)) put(dst + (j - 1) * bx * by, v[j], ep);
 #pragma unroll
-            for (int j = 1; j <= R; ++j) s0[o + (j + 1) * PS] = v[j];
+            for (int j = 1; j <= R; ++j)
+                if (keep >> j & 1u) s0[o + (j + 1) * PS] = v[j];
         }
         int left = kRounds;
         if (H > 0) {
@@ -712,12 +765,13 @@ __global__ void __launch_bounds__(NT, 1) k_res_pair(const __grid_constant__ Pres
         if (mine) {
             sweep(from, 1, R);
 #pragma unroll
-            for (int j = 1; j <= R; ++j)
-                if (z0 + j - 1 < a.nz && ai[j] != 0.f) {
-                    const size_t i = (size_t)(z0 + j - 1) * sxy + i0;
+            for (int j = 1; j <= R; ++j) {
+                const int i = (z0 + j - 1) * sxy + i0;
+                if (z0 + j - 1 < a.nz && written<F>(a, i, ai[j])) {
                     if (a.pprev) a.pprev[i] = from[o + (j + 1) * PS];
                     if (a.pout) a.pout[i] = v[j];
                 }
+            }
         }
     }
     epoch_end(a.ctl, base, (unsigned)a.n + 1u);
@@ -837,6 +891,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
     }
     // the column's coefficients (1/D is 0 on solid cells, whose b is not
     // theirs)
+    unsigned walls = 0;
     float A[6][R], d0[R], d12[kShared ? 1 : 2][kShared ? 1 : R], bb[kShared ? 1 : 3][kShared ? 1 : R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -846,6 +901,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
         for (int f = 0; f < 6; ++f) A[f][r] = in ? __ldg(a.A + f * N + i) : 0.f;
         d0[r] = in ? __ldg(a.iD + i) : 0.f;
         const bool fluid = d0[r] != 0.f;
+        if (own && !fluid) walls |= 1u << r;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const float v = fluid && a.bv ? __ldg(a.bv + c * N + i) : 0.f;
@@ -873,12 +929,20 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
                       : kShared ? priv[((2 + c) * R + r) * NT + tid] : d12[kShared ? 0 : (c > 0 ? c - 1 : 0)][kShared ? 0 : r];
         return d * (acc + rhs);
     };
+    const bool any_walls = __any_sync(0xffffffffu, walls != 0);
     float v0[3], vT[3];
     auto ends = [&]() {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             v0[c] = cell(c, 0, u[c][1], hd[c]);
             vT[c] = cell(c, R - 1, hu[c], u[c][R - 2]);
+        }
+        if (any_walls) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (walls & 1u) v0[c] = 0.f;
+                if (walls >> (R - 1) & 1u) vT[c] = 0.f;
+            }
         }
     };
     auto middle = [&]() {
@@ -894,6 +958,10 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
             }
             u[c][0] = v0[c];
             u[c][R - 1] = vT[c];
+        }
+        if (any_walls) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) clear_walls<1, R - 2>(walls, u[c]);
         }
     };
     auto emit = [&](float* out) {
@@ -1139,7 +1207,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel_wide(const __grid_constant__ 
                 acc += A[3][r] * cu[o0 - bx + k];
                 acc += A[4][r] * up;
                 acc += A[5][r] * bel[c];
-                v[c] = w[c == 0 ? 0 : 3 + c] * (acc + w[1 + c]);
+                v[c] = w[0] != 0.f ? w[c == 0 ? 0 : 3 + c] * (acc + w[1 + c]) : 0.f;
                 bel[c] = cen[c];
                 if (j > 0) cen[c] = up;
             }
