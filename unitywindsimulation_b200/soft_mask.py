@@ -43,13 +43,18 @@ class SoftBuildings:
         return dataclasses.replace(self, heights=np.asarray(heights, dtype=np.float64).copy())
 
     def _window(self, i: int, nx: int, nz: int):
-        """Index ranges (zlo, zhi, xlo, xhi) holding every cell of footprint i."""
+        """Index ranges (zlo, zhi, xlo, xhi) holding every cell of footprint i:
+        the bounding box of its corners, or the whole grid where a corner is
+        not finite (a strip or half plane without an end)."""
         x0, x1, z0, z1 = self.footprints[i]
         cx, cz = nx / 2.0, nz / 2.0
         th = np.radians(self.angle_deg)
         c, s = np.cos(th), np.sin(th)
-        xs = [cx + (x - cx) * c - (z - cz) * s for x in (x0, x1) for z in (z0, z1)]
-        zs = [cz + (x - cx) * s + (z - cz) * c for x in (x0, x1) for z in (z0, z1)]
+        with np.errstate(invalid="ignore", over="ignore"):
+            xs = [cx + (x - cx) * c - (z - cz) * s for x in (x0, x1) for z in (z0, z1)]
+            zs = [cz + (x - cx) * s + (z - cz) * c for x in (x0, x1) for z in (z0, z1)]
+        if not np.all(np.isfinite(xs + zs)):
+            return 0, nz, 0, nx
         lo = lambda v: max(0, int(np.floor(min(v))) - 1)  # noqa: E731
         hi = lambda v, n: max(lo(v), min(n, int(np.ceil(max(v))) + 1))  # noqa: E731
         return lo(zs), hi(zs, nz), lo(xs), hi(xs, nx)
