@@ -1241,6 +1241,7 @@ int wf_adj_step_vjp(wf_adjoint* a, int phases, const float* ubar_out, const floa
     wf_solver* h = a->h;
     WFA_CUDA(cudaSetDevice(h->device));
     WFA_CUDA(cudaStreamSynchronize(h->st));
+    wf::steps_end(h);
     const size_t N = a->N, v = 3 * N * sizeof(float), s = N * sizeof(float);
     Tape& t = a->tapes[0];
     // the solver's current state is the step input
@@ -1267,6 +1268,7 @@ int wf_adj_step_forward(wf_adjoint* a, int phases, float* u_out, float* p_out) {
     wf_solver* h = a->h;
     WFA_CUDA(cudaSetDevice(h->device));
     WFA_CUDA(cudaStreamSynchronize(h->st));
+    wf::steps_end(h);
     Tape& t = a->tapes[0];
     const int st = record_step(a, t, h->vb[h->iT], h->pr, phases);
     if (st != WF_OK) return st;
@@ -1290,6 +1292,7 @@ int wf_adj_gradient(wf_adjoint* a, const wf_objective* obj, int n_steps, int che
         return adj_fail(a, WF_ERR_UNSUPPORTED, "inflow gradients need the log inflow with inflow_ustar > 0");
     WFA_CUDA(cudaSetDevice(h->device));
     WFA_CUDA(cudaStreamSynchronize(h->st));
+    wf::steps_end(h);
     const size_t N = a->N, v = 3 * N * sizeof(float), s = N * sizeof(float);
     const int area = (obj->x1 - obj->x0) * (obj->z1 - obj->z0);
     const float w = 1.f / (float)(obj->window * area);
@@ -1382,6 +1385,7 @@ int wf_adj_gradient(wf_adjoint* a, const wf_objective* obj, int n_steps, int che
                                                   h->vb[h->iT], nullptr, a->dJ);
     }
     WFA_CUDA(cudaStreamSynchronize(h->st));
+    wf::steps_end(h);
     int rs = WF_OK;
     for (int j = 0; j < R; ++j) {
         const float* ui = j == 0 ? h->vb[h->iT] : a->tapes[j - 1].uout;

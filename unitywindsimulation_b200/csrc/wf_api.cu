@@ -11,6 +11,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -138,7 +139,7 @@ void free_all(wf_solver* h) {
     if (h->st) cudaStreamDestroy(h->st);
 }
 
-int sync(wf_solver* h) {
+int wait(wf_solver* h) {
     WF_CUDA(cudaStreamSynchronize(h->st));
     if (h->hstat && *(volatile int*)h->hstat) {
         *(volatile int*)h->hstat = 0;
@@ -146,6 +147,12 @@ int sync(wf_solver* h) {
                        "a bounded wait of a Jacobi loop's kernel ran out; the fields are not valid");
     }
     return WF_OK;
+}
+
+int sync(wf_solver* h) {
+    const int s = wait(h);
+    wf::steps_end(h);
+    return s;
 }
 
 // Makes velFieldLastIter a real buffer again (copy of velFieldLastTime).
@@ -204,7 +211,7 @@ int do_vel_precompute(wf_solver* h) {
 
 int read_residual(wf_solver* h, double* out) {
     WF_CUDA(cudaMemcpyAsync(h->hsum, h->dsum, sizeof(double), cudaMemcpyDeviceToHost, h->st));
-    WF_TRY(sync(h));
+    WF_TRY(wait(h));  // within a step: its handle's steps go on
     *out = h->hsum[0];
     return WF_OK;
 }
@@ -286,7 +293,7 @@ int do_pres_sweeps(wf_solver* h, int n, bool allow_fast) {
         WF_TRY(wf::pres_sweeps_fast(h, n, /*piso=*/false));
         return WF_OK;
     }
-    if (allow_fast && !resid && n >= 2 && wf::loops_on_chip(h, h->res.nupres_alone()) &&
+    if (allow_fast && !resid && n >= 2 && wf::loops_on_chip(h, wf::nupres_plan(h)) &&
         wf::pres_sweeps_on_chip(h, n, true, !h->in_step))
         return WF_OK;
     // with residual checks: the sweeps up to the next one on chip, in the
@@ -442,13 +449,20 @@ void set_roles(wf_solver* h, const wf_solver::RoleKey& k) {
 
 // Runs one step, replaying a cached CUDA graph when the handle is in its
 // steady state (iter_alias and pc_zero set, no residual reads).
-int run_step(wf_solver* h) {
+int run_step_as(wf_solver* h) {
     if (!wf::step_graphable(h)) return wf::run_step_eager(h);
     const wf_solver::GraphEntry* ent = nullptr;
     WF_TRY(wf::ensure_step_graph(h, &ent));
     WF_CUDA(cudaGraphLaunch(ent->exec, h->st));
     wf::commit_graph_step(h, *ent);
     return WF_OK;
+}
+int run_step(wf_solver* h) {
+    wf::steps_begin(h);
+    h->company = wf::beside_others(h) ? wf_solver::kBeside : wf_solver::kAlone;
+    const int s = run_step_as(h);
+    h->company = wf_solver::kAlone;
+    return s;
 }
 
 int check_finite(wf_solver* h) {
@@ -503,6 +517,53 @@ float* field_ptr(wf_solver* h, int field, size_t* points, int* comps) {
 
 namespace wf {
 
+namespace {
+// By device: handles with steps in flight, all handles, and how often a handle has begun.
+constexpr int kDevices = 64;
+std::atomic<int> g_pending[kDevices], g_handles[kDevices];
+std::atomic<long long> g_begun[kDevices];
+int slot_of(const wf_solver* h) { return h->device % kDevices; }
+}  // namespace
+
+void steps_begin(wf_solver* h) {
+    h->rb_stepped = true;
+    if (h->pending) return;
+    h->beside_begin = g_pending[slot_of(h)].fetch_add(1, std::memory_order_relaxed);
+    h->begin_ticket = g_begun[slot_of(h)].fetch_add(1, std::memory_order_relaxed);
+    h->pending = true;
+}
+void steps_end(wf_solver* h) {
+    if (!h->pending) return;
+    g_pending[slot_of(h)].fetch_sub(1, std::memory_order_relaxed);
+    // those in flight when it began and those that have begun since, no more than there are
+    const long long since = g_begun[slot_of(h)].load(std::memory_order_relaxed) - h->begin_ticket - 1;
+    const int others = std::max(g_handles[slot_of(h)].load(std::memory_order_relaxed) - 1, 0);
+    h->beside_seen = (int)std::min<long long>(h->beside_begin + since, others);
+    h->pending = false;
+}
+void count_handle(const wf_solver* h, int by) { g_handles[slot_of(h)].fetch_add(by, std::memory_order_relaxed); }
+namespace {
+// How many other handles make the splits beside others the faster ones: one where these
+// hold so little of the GPU that they cost nothing, else two (with one, of 0.1 M cells,
+// 0.33 ms a round of steps with the lone splits against 0.56).  0: the step has no such
+// splits (a residual-checked step launches its momentum sweeps one by one and was never
+// slower side by side).
+int company_needed(const wf_solver* h) {
+    const ResPlan &p = h->nonuniform ? h->res.nupres_beside : h->res.pres_beside, &v = h->res.vel_beside;
+    if (!h->resident || h->cfg.calc_residual || !shares(h, p) || !shares(h, v)) return 0;
+    return 8 * std::max(p.boxes(), v.boxes()) <= h->num_sms ? 1 : 2;
+}
+}  // namespace
+bool beside_others(const wf_solver* h) {
+    const int need = company_needed(h);
+    const int others = g_pending[slot_of(h)].load(std::memory_order_relaxed) - (h->pending ? 1 : 0);
+    return need > 0 && std::max(others, h->beside_seen) >= need;
+}
+bool may_run_beside(const wf_solver* h) {
+    const int need = company_needed(h);
+    return need > 0 && g_handles[slot_of(h)].load(std::memory_order_relaxed) > need;
+}
+
 bool step_graphable(const wf_solver* h) {
     return h->cfg.use_graph && !h->cfg.calc_residual && h->iter_alias && h->pc_zero;
 }
@@ -516,7 +577,7 @@ int run_step_eager(wf_solver* h) {
 
 int ensure_step_graph(wf_solver* h, const wf_solver::GraphEntry** out) {
     const auto key = role_key(h);
-    auto& graphs = h->in_batch ? h->batch_graphs : h->graphs;
+    auto& graphs = h->step_graphs();
     auto it = graphs.find(key);
     if (it == graphs.end()) {
         cudaGraph_t g = nullptr;
@@ -545,7 +606,7 @@ int ensure_step_graph(wf_solver* h, const wf_solver::GraphEntry** out) {
         ent.graph = g;
         ent.kernels = nk;
         ent.after = after;
-        if (!h->in_batch) e = cudaGraphInstantiate(&ent.exec, g, 0);  // a batch clones the graph into its own
+        if (h->company != wf_solver::kBatch) e = cudaGraphInstantiate(&ent.exec, g, 0);  // a batch clones the graph
         if (e != cudaSuccess) {
             cudaGraphDestroy(g);
             h->err = std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e);
@@ -609,7 +670,7 @@ void commit_graph_step(wf_solver* h, const wf_solver::GraphEntry& e) {
 }
 
 void drop_graphs(wf_solver* h) {
-    for (auto* m : {&h->graphs, &h->batch_graphs}) {
+    for (auto* m : {&h->graphs, &h->batch_graphs, &h->beside_graphs}) {
         for (auto& kv : *m) {
             if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
             if (kv.second.graph) cudaGraphDestroy(kv.second.graph);
@@ -779,6 +840,7 @@ int wf_create(const wf_config* cfg, int device, wf_solver** out) {
     if ((s = wf_init_vel_pres_fields(h)) != WF_OK) return fail(s);
     if ((s = wf_set_fixed_value_vel_bnd_cond(h, h->wind)) != WF_OK) return fail(s);
     if ((s = sync(h)) != WF_OK) return fail(s);
+    wf::count_handle(h, 1);
     *out = h;
     return WF_OK;
 }
@@ -787,6 +849,8 @@ int wf_destroy(wf_solver* h) {
     if (!h) return WF_ERR_INVALID_ARG;
     cudaSetDevice(h->device);
     cudaStreamSynchronize(h->st);
+    wf::steps_end(h);
+    wf::count_handle(h, -1);
     free_all(h);
     delete h;
     return WF_OK;
@@ -927,18 +991,21 @@ int wf_prepare_graphs(wf_solver* h) {
     WF_CUDA(cudaSetDevice(h->device));
     if (!wf::step_graphable(h)) return WF_OK;  // not in the replay state yet
     const auto start = role_key(h);
-    for (int i = 0; i < 64; ++i) {
-        const wf_solver::GraphEntry* e = nullptr;
-        const int st = wf::ensure_step_graph(h, &e);
-        if (st != WF_OK) {
-            set_roles(h, start);
-            return st;
+    int st = WF_OK;
+    auto capture = [&](wf_solver::Company company) {
+        h->company = company;
+        for (int i = 0; i < 64 && st == WF_OK; ++i) {
+            const wf_solver::GraphEntry* e = nullptr;
+            st = wf::ensure_step_graph(h, &e);
+            if (st == WF_OK) set_roles(h, e->after);
+            if (role_key(h) == start) break;
         }
-        set_roles(h, e->after);
-        if (role_key(h) == start) break;
-    }
-    set_roles(h, start);
-    return WF_OK;
+        set_roles(h, start);
+        h->company = wf_solver::kAlone;
+    };
+    capture(wf_solver::kAlone);
+    if (st == WF_OK && wf::may_run_beside(h)) capture(wf_solver::kBeside);
+    return st;
 }
 
 namespace {
@@ -1075,6 +1142,7 @@ int wf_readback_wait(wf_solver* h) {
     WF_CUDA(cudaSetDevice(h->device));
     h->rb_pending = false;
     WF_CUDA(cudaEventSynchronize(h->ev_done));
+    if (!h->rb_stepped) wf::steps_end(h);
     return WF_OK;
 }
 
@@ -1107,6 +1175,7 @@ int wf_readback_begin(wf_solver* h, float* vel, float* pres, int layout) {
     WF_CUDA(cudaMemcpyAsync(pres, psnap, sizeof(float) * N, cudaMemcpyDeviceToHost, h->cst));
     WF_CUDA(cudaEventRecord(h->ev_done, h->cst));
     h->rb_pending = true;
+    h->rb_stepped = false;
     return WF_OK;
 }
 

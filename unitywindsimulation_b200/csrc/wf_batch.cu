@@ -442,9 +442,9 @@ int ensure_batch_graph(wf_batch* b, const wf_batch::Entry** out) {
         for (size_t i = 0; i < b->s.size(); ++i) {
             wf_solver* h = b->s[i];
             const wf_solver::GraphEntry* ge = nullptr;
-            h->in_batch = b->s.size() > 1;
+            h->company = b->s.size() > 1 ? wf_solver::kBatch : wf_solver::kAlone;
             const int st = wf::ensure_step_graph(h, &ge);
-            h->in_batch = false;
+            h->company = wf_solver::kAlone;
             if (st != WF_OK) {
                 cudaGraphDestroy(parent);
                 return fail(b, st, "capturing a case's step failed: " + h->err);
@@ -521,8 +521,10 @@ int wf_batch_step(wf_batch* b, int n_steps) {
     if (cudaSetDevice(b->device) != cudaSuccess) return fail(b, WF_ERR_CUDA, "cudaSetDevice failed");
     // Work still queued on a case's own stream (an inflow-plane upload, an
     // asynchronous step) finishes before the batch touches the case.
-    for (wf_solver* h : b->s)
+    for (wf_solver* h : b->s) {
         if (cudaStreamSynchronize(h->st) != cudaSuccess) return fail(b, WF_ERR_CUDA, "case stream failed");
+        wf::steps_end(h);
+    }
     // Cases not yet in the graph-replay state (first step after an init or
     // a field write) take one eager step on their own stream first.
     bool any_eager = false;
@@ -530,9 +532,9 @@ int wf_batch_step(wf_batch* b, int n_steps) {
         if (!h->cfg.use_graph || h->cfg.calc_residual)
             return fail(b, WF_ERR_UNSUPPORTED, "batched cases need use_graph and no residual checks");
         if (!wf::step_graphable(h) && n_steps > 0) {
-            h->in_batch = b->s.size() > 1;
+            h->company = b->s.size() > 1 ? wf_solver::kBatch : wf_solver::kAlone;
             const int st = wf::run_step_eager(h);
-            h->in_batch = false;
+            h->company = wf_solver::kAlone;
             if (st != WF_OK) return fail(b, st, "eager step failed: " + h->err);
             any_eager = true;
         }
@@ -712,6 +714,7 @@ int wf_set_blocking(wf_solver* h, int pres_k, int vel_k) {
     }
     if (cudaSetDevice(h->device) != cudaSuccess) return WF_ERR_CUDA;
     cudaStreamSynchronize(h->st);
+    wf::steps_end(h);
     wf::drop_graphs(h);  // captured steps encode the old depths
     h->pres_k = pres_k;
     h->vel_k = vel_k;
@@ -727,6 +730,7 @@ int wf_set_loops(wf_solver* h, int mode) {
     }
     if (cudaSetDevice(h->device) != cudaSuccess) return WF_ERR_CUDA;
     cudaStreamSynchronize(h->st);
+    wf::steps_end(h);
     wf::drop_graphs(h);  // captured steps encode the old loops
     h->resident = mode == WF_LOOPS_AUTO;
     return WF_OK;
@@ -741,6 +745,7 @@ int wf_set_tiles(wf_solver* h, int pres_rows, int vel_bx, int vel_by, int vel_bz
     }
     if (cudaSetDevice(h->device) != cudaSuccess) return WF_ERR_CUDA;
     cudaStreamSynchronize(h->st);
+    wf::steps_end(h);
     wf::drop_graphs(h);  // captured steps encode the old tiles
     h->pres_ty = pres_rows;
     h->vel_blk[0] = vel_bx;

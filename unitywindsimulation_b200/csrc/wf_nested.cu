@@ -120,6 +120,7 @@ extern "C" int wf_init_from_background(wf_solver* h, const wf_solver* bg, const 
     for (int k = 0; k < 3 && e == cudaSuccess; ++k)
         e = cudaMemsetAsync(h->pcb[k], 0, sizeof(float) * h->P.N, h->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
+    wf::steps_end(h);
     if (e != cudaSuccess) {
         h->err = std::string("init from background: ") + cudaGetErrorString(e);
         return WF_ERR_CUDA;

@@ -1332,9 +1332,9 @@ VelKernel vel_kernel(int R) {
 // 14, 3.4 with 16: the cells of a thread weigh most (a warp works through
 // them one after another), then the warps, then the halo.
 // loop: whose limits the split has to keep.
-// shared: beside other cases' loops the product of a sweep's time and the
-// multiprocessors it holds counts instead, so that as many loops as possible
-// run at once.
+// part > 0: beside other loops the product of a sweep's time and the
+// multiprocessors it holds, `part` at least, counts instead, so that as many loops as
+// possible run at once.
 enum class Loop { kPres, kVel, kVelWide, kPair };
 bool fits(const ResPlan& pl, Loop loop) {
     if (rim_of(pl) + 4 > NT) return false;
@@ -1347,7 +1347,7 @@ bool fits(const ResPlan& pl, Loop loop) {
            (loop == Loop::kPres || fetches_of(pl) <= fetch_max(pl.bz));
 }
 template <size_t M>
-ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], Loop loop = Loop::kPres, bool shared = false) {
+ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], Loop loop = Loop::kPres, int part = 0) {
     ResPlan best;
     double cost = 1e30;
     sms = std::min(sms, kMaxBoxes);
@@ -1366,7 +1366,7 @@ ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], Loop loop = Loop
                 if (!fits(pl, loop)) continue;
                 const double halo = 2.0 * ((px > 1 ? by * R : 0) + (py > 1 ? bx * R : 0) + (pz > 1 ? bx * by : 0));
                 double c = R * (60.0 + 0.6 * (inner0_of(pl) / 32 + (inner_of(pl) + 31) / 32)) + 0.03 * halo;
-                if (shared) c = (500.0 + c) * pl.boxes();
+                if (part > 0) c = (500.0 + c) * std::max(pl.boxes(), part);
                 if (c < cost) {
                     cost = c;
                     best = pl;
@@ -1428,8 +1428,14 @@ int resident_setup(const Resident& r) {
     }
     if (r.nupres.bz > 0) opt_in(pres_kernel<Form::kStretched, false>(r.nupres.bz));
     if (r.pres_shared.bz > 0) opt_in(pres_kernel<Form::kPasses, false>(r.pres_shared.bz));
+    if (r.pres_beside.bz > 0)
+        opt_in(r.pres_beside.pair ? pair_kernel<Form::kPasses>(r.pres_beside.bz)
+                                  : pres_kernel<Form::kPasses, false>(r.pres_beside.bz));
+    if (r.nupres_beside.bz > 0)
+        opt_in(r.nupres_beside.pair ? pair_kernel<Form::kStretched>(r.nupres_beside.bz)
+                                    : pres_kernel<Form::kStretched, false>(r.nupres_beside.bz));
     if (r.vel.bz > 0) opt_in(vel_kernel<true>(r.vel.bz));
-    for (const ResPlan& p : {r.vel, r.vel_shared})
+    for (const ResPlan& p : {r.vel, r.vel_shared, r.vel_beside})
         if (p.bz > 0) opt_in(vel_kernel<false>(p.bz));
     return e == cudaSuccess ? WF_OK : WF_ERR_CUDA;
 }
@@ -1441,16 +1447,24 @@ void resident_plan(const Params& P, int sms, Resident* r) {
     r->nupres2 = r->pres2;
     r->vel = make_plan(P, sms, kVelR, Loop::kVel);
     if (r->vel.bz == 0) r->vel = make_plan(P, sms, kVelWideR, Loop::kVelWide);
-    r->pres_shared = make_plan(P, sms, kPresR, Loop::kPres, true);
-    r->vel_shared = make_plan(P, sms, kVelR, Loop::kVel, true);
+    r->pres_shared = make_plan(P, sms, kPresR, Loop::kPres, 1);
+    r->vel_shared = make_plan(P, sms, kVelR, Loop::kVel, 1);
+    // Beside other handles: an eighth of the multiprocessors costs nothing yet.
+    const int part = std::max(sms / 8, 1);
+    const ResPlan pair = make_plan(P, sms, kPairR, Loop::kPair, part);
+    auto better = [&](const ResPlan& p) { return pair.bz > 0 && pair.boxes() <= std::max(p.boxes(), part) ? pair : p; };
+    r->pres_beside = better(make_plan(P, sms, kPresR, Loop::kPres, part));
+    r->nupres_beside = better(make_plan(P, sms, kNuPresR, Loop::kPres, part));
+    r->vel_beside = make_plan(P, sms, kVelR, Loop::kVel, part);
 }
 
 void resident_alloc(Resident* r, cudaStream_t st) {
     // both parities of the pressure packets, then of the momentum packets
     // (apart: a momentum packet's words must not be read as pressure
     // packets), then the epoch words
-    const size_t np = 2 * std::max({packets(r->pres), packets(r->nupres), packets(r->pres2), packets(r->pres_shared)}),
-                 nv = 2 * std::max(packets(r->vel), packets(r->vel_shared));
+    const size_t np = 2 * std::max({packets(r->pres), packets(r->nupres), packets(r->pres2), packets(r->pres_shared),
+                                    packets(r->pres_beside), packets(r->nupres_beside)}),
+                 nv = 2 * std::max({packets(r->vel), packets(r->vel_shared), packets(r->vel_beside)});
     if (np + nv == 0 || r->work.pk) return;
     const size_t bytes = np * sizeof(unsigned long long) + nv * sizeof(Packet3) + 16 +
                          streamed(r->vel) * sizeof(float);

@@ -31,7 +31,8 @@ struct Resident {
     ResPlan nupres;    // non-uniform pressure loop
     ResPlan pres2, nupres2;  // the same, two sweeps a halo trip, where that is faster
     ResPlan vel;       // momentum loop
-    ResPlan pres_shared, vel_shared;  // the same beside other cases' loops: fewest multiprocessors
+    ResPlan pres_shared, vel_shared;  // the same beside the cases of a batch: fewest multiprocessors
+    ResPlan pres_beside, nupres_beside, vel_beside;  // beside a few other handles' loops
     ResWork work;
     const ResPlan& pres_alone() const { return pres2.bz > 0 ? pres2 : pres; }
     const ResPlan& nupres_alone() const { return nupres2.bz > 0 ? nupres2 : nupres; }

@@ -103,7 +103,17 @@ struct wf_solver {
     // 0: the pass kernels (wf_set_loops, an explicit depth or tile, WF_RESIDENT=0)
     int resident = 1;
     wf::Resident res;
-    bool in_batch = false;    // the step being enqueued runs beside other cases' steps
+    // what the step being enqueued runs beside: nothing, other handles' steps on their
+    // own streams, or the other cases of a batch
+    enum Company { kAlone, kBeside, kBatch };
+    Company company = kAlone;
+    // steps enqueued and not waited for yet; how many other handles of the device had
+    // such steps when they were enqueued, and up to when they were waited for
+    // (steps_begin, steps_end)
+    bool pending = false;
+    int beside_begin = 0, beside_seen = 0;
+    long long begin_ticket = 0;
+    bool rb_stepped = false;  // a step was enqueued after the readback in flight
     int vel_blk[3] = {32, 4, 2};  // block of the four-cell momentum sweep (256 threads)
     int num_sms = 148;        // multiprocessors of the device
     int pdl = 1;              // programmatic dependent launch in the non-uniform grid's sweep chains
@@ -124,11 +134,37 @@ struct wf_solver {
         long long kernels = 0;
     };
     std::map<RoleKey, GraphEntry> graphs;
-    std::map<RoleKey, GraphEntry> batch_graphs;  // the same for steps beside other cases (exec unused)
+    std::map<RoleKey, GraphEntry> batch_graphs;   // the same for steps in a batch (exec unused)
+    std::map<RoleKey, GraphEntry> beside_graphs;  // and for steps beside other handles' steps
+    std::map<RoleKey, GraphEntry>& step_graphs() {
+        return company == kBatch ? batch_graphs : company == kBeside ? beside_graphs : graphs;
+    }
 };
 
 namespace wf {
 inline bool loops_on_chip(const wf_solver* h, const ResPlan& p) { return h->resident && h->dstat && h->res.ok(p); }
+// Handles whose steps run at the same time (step_async on their own streams, one
+// thread a handle, any mix): a loop on all multiprocessors waits until the other handles'
+// loops have left, so beside others a handle takes splits that leave at least half of
+// the multiprocessors to them, where there are such.  A handle knows its company by a
+// count per device of the handles with steps in flight: those it sees when it enqueues,
+// or those that its last steps ran beside (the first handle of a round sees none when it
+// enqueues).  The fields do not depend on it.  Ms for one step of each of 2 / 4 / 16
+// handles, passes, lone splits, now: 24 x 12 x 16 0.56 / 0.57 / 0.64, 0.29 / 0.57 / 2.22, 0.18 /
+// 0.19 / 0.27; 64 x 32 x 48 0.61 / 0.76 / 2.80, 0.33 / 0.68 / 2.80, 0.33 / 0.48 / 1.42; 72 x 40 x 72
+// 0.75 / 1.17 / 5.3, 0.47 / 0.97 / 4.0, 0.45 / 0.67 / 2.7; stretched 24 x 12 x 16 0.21 / 0.22 / 0.40,
+// 0.23 / 0.46 / 1.82, 0.13 / 0.14 / 0.21, 64 x 32 x 48 0.27 / 0.38 / 1.61, 0.27 / 0.56 / 2.29, 0.27 / 0.33 /
+// 1.24.  Larger grids keep the lone splits: 100 x 50 x 100 1.39 / 3.6 / - in passes, 0.85 / 1.81
+// / -.
+void steps_begin(wf_solver* h);
+void steps_end(wf_solver* h);  // nothing of the handle's stream is in flight any more
+bool beside_others(const wf_solver* h);
+// Counts a handle of the device in or out; whether there are others that it may yet
+// step beside (wf_prepare_graphs then captures both forms of its step).
+void count_handle(const wf_solver* h, int by);
+bool may_run_beside(const wf_solver* h);
+inline bool shares(const wf_solver* h, const ResPlan& p) { return p.bz > 0 && 2 * p.boxes() <= h->num_sms; }
+
 // The loops' splits: the fastest alone; beside the other cases of a batch the
 // one that holds the fewest multiprocessors for its time, where it leaves at
 // least half of them to the others.  A larger case keeps its pressure split for
@@ -139,19 +175,24 @@ inline bool loops_on_chip(const wf_solver* h, const ResPlan& p) { return h->resi
 // with lone momentum splits too (loops of more than half the GPU each wait for it
 // to empty).
 inline const ResPlan& pres_plan(const wf_solver* h) {
-    if (!h->in_batch) return h->res.pres_alone();
-    return 2 * h->res.pres_shared.boxes() <= h->num_sms ? h->res.pres_shared : h->res.pres;
+    if (h->company == wf_solver::kAlone) return h->res.pres_alone();
+    if (h->company == wf_solver::kBeside) return h->res.pres_beside;
+    return shares(h, h->res.pres_shared) ? h->res.pres_shared : h->res.pres;
+}
+inline const ResPlan& nupres_plan(const wf_solver* h) {
+    return h->company == wf_solver::kBeside ? h->res.nupres_beside : h->res.nupres_alone();
 }
 inline const ResPlan& vel_plan(const wf_solver* h) {
     static const ResPlan none;
-    if (!h->in_batch) return h->res.vel;
-    return 2 * h->res.vel_shared.boxes() <= h->num_sms ? h->res.vel_shared : none;
+    if (h->company == wf_solver::kAlone) return h->res.vel;
+    if (h->company == wf_solver::kBeside) return h->res.vel_beside;
+    return shares(h, h->res.vel_shared) ? h->res.vel_shared : none;
 }
 
 // Step-graph plumbing shared by the single-handle and the batched step.
 bool step_graphable(const wf_solver* h);
-// Captures (once per buffer-role assignment) the graph of one step from the
-// handle's current state without running it.
+// Captures (once per buffer-role assignment and company) the graph of one step from
+// the handle's current state without running it.
 int ensure_step_graph(wf_solver* h, const wf_solver::GraphEntry** out);
 // Applies the role rotation and counters of one replayed step.
 void commit_graph_step(wf_solver* h, const wf_solver::GraphEntry& e);

@@ -1086,7 +1086,7 @@ bool pres_sweeps_on_chip(wf_solver* h, int n, bool coef_done, bool keep_prev) {
     const size_t N = h->P.N;
     if (!h->nonuniform && !coef_done) pres_coef(h, /*piso=*/false);
     return pres_loop(h, keep_prev, [&](const float* in, float* out, float* prev) {
-        return h->nonuniform ? launch_res_nupres(h->P, h->st, h->res.nupres_alone(), h->res.work, h->nucoef, h->bp, in, out,
+        return h->nonuniform ? launch_res_nupres(h->P, h->st, nupres_plan(h), h->res.work, h->nucoef, h->bp, in, out,
                                                  prev, n, h->dstat)
                              : launch_res_pres(h->P, h->st, h->res.pres_alone(), h->res.work, h->pcoef, h->pcoef + 3 * N,
                                                h->bp, in, out, prev, nullptr, n, h->dstat, /*ordered=*/true);
