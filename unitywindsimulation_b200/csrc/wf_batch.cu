@@ -424,6 +424,17 @@ int fused_step(wf_batch* b) {
     return WF_OK;
 }
 
+// Chains of cases that run at the same time, and so what a case's step runs beside: on
+// one chain the cases run one after another, each with the GPU to itself (8 cases of 64 x
+// 32 x 48: 4.44 ms a step with the splits for company, 1.70 with the lone ones).
+int chains_of(const wf_batch* b) {
+    const int n = (int)b->s.size();
+    return b->width > 0 ? std::min(b->width, n) : n;
+}
+wf_solver::Company company_of(const wf_batch* b) {
+    return chains_of(b) > 1 ? wf_solver::kBatch : wf_solver::kAlone;
+}
+
 // Parent graph with one child-graph branch per case for the cases' current
 // buffer roles.
 int ensure_batch_graph(wf_batch* b, const wf_batch::Entry** out) {
@@ -437,12 +448,12 @@ int ensure_batch_graph(wf_batch* b, const wf_batch::Entry** out) {
         wf_batch::Entry ent;
         // Cases are dealt round-robin onto `width` chains; the chains run
         // concurrently, the cases of one chain one after another.
-        const int width = b->width > 0 ? std::min<int>(b->width, (int)b->s.size()) : (int)b->s.size();
+        const int width = chains_of(b);
         std::vector<cudaGraphNode_t> tail(width, nullptr);
         for (size_t i = 0; i < b->s.size(); ++i) {
             wf_solver* h = b->s[i];
             const wf_solver::GraphEntry* ge = nullptr;
-            h->company = b->s.size() > 1 ? wf_solver::kBatch : wf_solver::kAlone;
+            h->company = company_of(b);
             const int st = wf::ensure_step_graph(h, &ge);
             h->company = wf_solver::kAlone;
             if (st != WF_OK) {
@@ -532,7 +543,7 @@ int wf_batch_step(wf_batch* b, int n_steps) {
         if (!h->cfg.use_graph || h->cfg.calc_residual)
             return fail(b, WF_ERR_UNSUPPORTED, "batched cases need use_graph and no residual checks");
         if (!wf::step_graphable(h) && n_steps > 0) {
-            h->company = b->s.size() > 1 ? wf_solver::kBatch : wf_solver::kAlone;
+            h->company = company_of(b);
             const int st = wf::run_step_eager(h);
             h->company = wf_solver::kAlone;
             if (st != WF_OK) return fail(b, st, "eager step failed: " + h->err);
