@@ -481,6 +481,11 @@ int wf_set_blocking(wf_solver* h, int pres_k, int vel_k);
  * batches that contain the handle afterwards. */
 enum { WF_LOOPS_AUTO = 0, WF_LOOPS_PASSES = 1 };
 int wf_set_loops(wf_solver* h, int mode);
+/* How the handle's step runs one of its two Jacobi loops (`kernel`: WF_KERNEL_*) in the
+ * present mode: the blocks of its cooperative launch, the cells a thread owns and the
+ * sweeps a halo exchange, or 0, 0, 0 where it runs as passes.  beside != 0: while other
+ * handles of the device step at the same time. */
+int wf_get_loop_plan(const wf_solver* h, int kernel, int beside, int* blocks, int* cells, int* sweeps_per_trip);
 int wf_get_blocking(const wf_solver* h, int* pres_k, int* vel_k);
 /* Tile shapes of the Jacobi kernels: rows of the pressure multi-sweep tile
  * (32: 32 x 32 tiles, one block per SM; 16: 32 x 16 tiles, two blocks per

@@ -554,6 +554,7 @@ int company_needed(const wf_solver* h) {
     return 8 * std::max(p.boxes(), v.boxes()) <= h->num_sms ? 1 : 2;
 }
 }  // namespace
+bool has_beside_splits(const wf_solver* h) { return company_needed(h) > 0; }
 bool beside_others(const wf_solver* h) {
     const int need = company_needed(h);
     const int others = g_pending[slot_of(h)].load(std::memory_order_relaxed) - (h->pending ? 1 : 0);

@@ -747,6 +747,25 @@ int wf_set_loops(wf_solver* h, int mode) {
     return WF_OK;
 }
 
+int wf_get_loop_plan(const wf_solver* h, int kernel, int beside, int* blocks, int* cells, int* sweeps_per_trip) {
+    if (!h || !blocks || !cells || !sweeps_per_trip || (kernel != WF_KERNEL_PRES_SWEEP && kernel != WF_KERNEL_VEL_SWEEP))
+        return WF_ERR_INVALID_ARG;
+    const wf_config& c = h->cfg;
+    const bool split = beside && wf::has_beside_splits(h), vel = kernel == WF_KERNEL_VEL_SWEEP;
+    const wf::ResPlan& p = vel           ? split ? h->res.vel_beside : h->res.vel
+                           : h->nonuniform ? split ? h->res.nupres_beside : h->res.nupres_alone()
+                                           : split ? h->res.pres_beside : h->res.pres_alone();
+    // sweeps of the longest launch: with residual checks the momentum sweeps go one by one,
+    // the pressure sweeps from check to check after the first
+    const int n = vel ? c.calc_residual ? 1 : c.vel_iters
+                      : c.calc_residual ? std::min(c.pres_res_interval, c.pres_iters - 1) : c.pres_iters;
+    const bool chip = h->fast && n >= 2 && wf::loops_on_chip(h, p);
+    *blocks = chip ? p.boxes() : 0;
+    *cells = chip ? p.bz : 0;
+    *sweeps_per_trip = !chip ? 0 : p.pair ? 2 : 1;
+    return WF_OK;
+}
+
 int wf_set_tiles(wf_solver* h, int pres_rows, int vel_bx, int vel_by, int vel_bz) {
     if (!h) return WF_ERR_INVALID_ARG;
     if ((pres_rows != 32 && pres_rows != 16) || vel_bx < 1 || vel_by < 1 || vel_bz < 1 ||

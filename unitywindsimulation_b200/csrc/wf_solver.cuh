@@ -162,6 +162,7 @@ bool beside_others(const wf_solver* h);
 // Counts a handle of the device in or out; whether there are others that it may yet
 // step beside (wf_prepare_graphs then captures both forms of its step).
 void count_handle(const wf_solver* h, int by);
+bool has_beside_splits(const wf_solver* h);
 bool may_run_beside(const wf_solver* h);
 inline bool shares(const wf_solver* h, const ResPlan& p) { return p.bz > 0 && 2 * p.boxes() <= h->num_sms; }
 

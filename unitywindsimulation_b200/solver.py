@@ -287,6 +287,14 @@ class FvmSolverCuda:
         the default) or _lib.LOOPS_PASSES (wf_set_loops)."""
         self._check(self._lib.wf_set_loops(self._h, int(mode)))
 
+    def loop_plan(self, kernel: int, beside: bool = False):
+        """(blocks, cells a thread, sweeps a halo exchange) of the step's loop
+        on chip, (0, 0, 0) where it runs as passes; `beside`: while other
+        handles step at the same time (wf_get_loop_plan)."""
+        v = [c_int(0) for _ in range(3)]
+        self._check(self._lib.wf_get_loop_plan(self._h, int(kernel), int(beside), *map(byref, v)))
+        return tuple(x.value for x in v)
+
     def get_blocking(self):
         p, v = c_int(0), c_int(0)
         self._check(self._lib.wf_get_blocking(self._h, byref(p), byref(v)))
