@@ -9,7 +9,7 @@ wavefront's tile is 32 x 32 (one block per SM) or 32 x 16 (two per SM, more
 tiles on small grids); the four-cell momentum sweep's block is one of
 VEL_BLOCKS.  The tuner times every depth and tile on the case itself with CUDA
 events (wf_time_kernel, cold L2) and keeps the fastest, cached as JSON keyed
-by device and grid so a grid size is tuned once.  Results never depend on the
+by device, grid and sweep counts so a configuration is tuned once.  Results never depend on the
 depth or tile; only speed does.  tune_batch picks the batched form's mode
 (child graphs or persistent loops) and, for graphs, the chain width.
 """
@@ -27,9 +27,18 @@ VEL_DEPTHS = (1, 2)
 VEL_BLOCKS = ((32, 4, 2), (32, 8, 1), (16, 8, 2), (64, 2, 2), (8, 8, 4))
 
 
+def _sweeps(cfg):
+    """(momentum, pressure) sweeps of one step."""
+    loops = 1 + (cfg.piso_correctors if cfg.solver_type == _lib.SOLVER_PISO else 0)
+    return cfg.vel_iters, cfg.pres_iters * loops
+
+
 def _key(solver, device_name: str) -> str:
+    # the sweep counts too: a loop on chip reads its coefficients once, so its
+    # time a sweep depends on them, and the two loops share one choice
     c = solver.cfg
-    return f"{device_name}|{c.nx}x{c.ny}x{c.nz}"
+    v, p = _sweeps(c)
+    return f"{device_name}|{c.nx}x{c.ny}x{c.nz}|{v}v{c.pres_iters}p{p}"
 
 
 def _device_name(device: int = 0) -> str:
@@ -88,8 +97,10 @@ def tune_batch(batch, widths=(1, 2, 4, 0), steps: int = 2, modes=None) -> dict:
 
 def tune(solver, cache_path: str | None = DEFAULT_CACHE, reps: int = 5, device_name: str | None = None) -> dict:
     """Picks and applies the fastest blocking depths and tile shapes for
-    `solver`'s grid, and whether its loops run on chip.  Returns {"loops", "pres_k", "pres_rows", "vel_k", "vel_block",
-    "pres_us_per_sweep", "vel_us_per_sweep", "cached"}."""
+    `solver`'s grid, and whether its loops run on chip: by the time of a step's
+    sweeps, momentum and pressure together.  Returns {"loops", "pres_k",
+    "pres_rows", "vel_k", "vel_block", "pres_us_per_sweep",
+    "vel_us_per_sweep", "cached"}, the times of what then runs."""
     name = device_name or _device_name()
     key = _key(solver, name)
     cache = load_cache(cache_path) if cache_path else {}
@@ -103,11 +114,14 @@ def tune(solver, cache_path: str | None = DEFAULT_CACHE, reps: int = 5, device_n
     saved = solver.get_blocking()
     _, vblk0 = solver.get_tiles()
     best_p, best_v = None, None
-    # the loop that keeps the grid on chip, where it fits (one launch is then
-    # the whole loop, more sweeps than any pass)
+    # the loops that keep the grid on chip, where it fits (one launch is then
+    # the whole loop)
     solver.set_loops(_lib.LOOPS_AUTO)
-    ms, _, sweeps = solver.time_kernel(_lib.KERNEL_PRES_SWEEP, reps=reps, flush_l2=True)
-    chip_us = ms * 1e3 / sweeps if sweeps > max(PRES_DEPTHS) else None
+    chip = {}
+    for kernel in (_lib.KERNEL_PRES_SWEEP, _lib.KERNEL_VEL_SWEEP):
+        if solver.loop_plan(kernel)[0] > 0:
+            ms, _, sweeps = solver.time_kernel(kernel, reps=reps, flush_l2=True)
+            chip[kernel] = ms * 1e3 / sweeps
     for rows in PRES_ROWS:
         solver.set_tiles(rows, vblk0)
         for k in PRES_DEPTHS:
@@ -127,11 +141,16 @@ def tune(solver, cache_path: str | None = DEFAULT_CACHE, reps: int = 5, device_n
                 best_v = (k, blk, us)
     solver.set_blocking(best_p[0], best_v[0])
     solver.set_tiles(best_p[1], best_v[1])
-    on_chip = chip_us is not None and chip_us < best_p[2]
+    nv, np_ = _sweeps(solver.cfg)
+    passes = best_p[2], best_v[2]
+    mixed = chip.get(_lib.KERNEL_PRES_SWEEP, best_p[2]), chip.get(_lib.KERNEL_VEL_SWEEP, best_v[2])
+    step = lambda us: np_ * us[0] + nv * us[1]  # noqa: E731
+    on_chip = bool(chip) and step(mixed) < step(passes)
+    us = mixed if on_chip else passes
     loops = _lib.LOOPS_AUTO if on_chip else _lib.LOOPS_PASSES
     solver.set_loops(loops)
     e = {"loops": loops, "pres_k": best_p[0], "pres_rows": best_p[1], "vel_k": best_v[0], "vel_block": list(best_v[1]),
-         "pres_us_per_sweep": chip_us if on_chip else best_p[2], "vel_us_per_sweep": best_v[2]}
+         "pres_us_per_sweep": us[0], "vel_us_per_sweep": us[1]}
     if cache_path:
         cache[key] = e
         save_cache(cache_path, cache)
