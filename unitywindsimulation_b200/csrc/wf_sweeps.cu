@@ -1183,19 +1183,20 @@ int time_kernel(wf_solver* h, int which, int reps, bool flush, float* ms, double
     const bool res_v = which == WF_KERNEL_VEL_SWEEP && loops_on_chip(h, vel_plan(h)) && h->cfg.vel_iters >= 2;
     const int kv = res_v ? h->cfg.vel_iters : std::min(std::max(h->vel_k, 1), 2);
     const int kp = res_p ? h->cfg.pres_iters : std::min(std::max(h->pres_k, 1), 4);
-    for (int r = 0; r < reps; ++r) {
+    cudaError_t err = cudaSuccess;
+    for (int r = 0; r < reps && err == cudaSuccess; ++r) {
         if (flush) k_flush_read<<<148 * 4, 512, 0, h->st>>>((const float4*)fbuf, flush_bytes / 16, (float*)fbuf);
         cudaEventRecord(e0, h->st);
         if (which == WF_KERNEL_VEL_SWEEP) {
             if (res_v)
-                launch_res_vel(P, h->st, vel_plan(h), h->res.work, h->vcoef, h->vcoef + 6 * N, h->bv, a, b, nullptr, kv,
-                               h->dstat);
+                err = launch_res_vel(P, h->st, vel_plan(h), h->res.work, h->vcoef, h->vcoef + 6 * N, h->bv, a, b,
+                                     nullptr, kv, h->dstat);
             else if (kv > 1) launch_vmsweep(h, kv, a, b, nullptr);
             else launch_vel_sweep_fast(h, a, b);
         } else {
             if (res_p)
-                launch_res_pres(P, h->st, pres_plan(h), h->res.work, h->pcoef, h->pcoef + 3 * N, rhs, a, b, nullptr,
-                                nullptr, kp, h->dstat);
+                err = launch_res_pres(P, h->st, pres_plan(h), h->res.work, h->pcoef, h->pcoef + 3 * N, rhs, a, b,
+                                      nullptr, nullptr, kp, h->dstat);
             else if (kp > 1) launch_msweep(h, kp, rhs, a, b, nullptr);
             else launch_pres_sweep_fast(h, rhs, a, b);
         }
@@ -1209,7 +1210,8 @@ int time_kernel(wf_solver* h, int which, int reps, bool flush, float* ms, double
     g_launches = saved;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    cudaError_t err = cudaGetLastError();
+    // a refused launch is no time (its launcher has cleared the error)
+    if (err == cudaSuccess) err = cudaGetLastError();
     cudaStreamSynchronize(h->st);
     cudaFree(scratch);
     if (fbuf) cudaFree(fbuf);
