@@ -472,6 +472,13 @@ int wf_stage_wait_selftest(wf_solver* h, int short_stage, double timeout_ms, int
  * package).  Drops the handle's captured step graphs; rebuild batches that
  * contain the handle afterwards. */
 int wf_set_blocking(wf_solver* h, int pres_k, int vel_k);
+/* Self-test of the bounded waits of the loops on chip (wf_set_loops): runs a short loop
+ * of `kernel` (WF_KERNEL_*) with the handle's split over scratch iterates, each wait limited to
+ * `rounds` polls; block silent_block (-1: none) sends no halo, so that its neighbours' waits run
+ * out.  *status is what wf_sync would then return (WF_OK or WF_ERR_TIMEOUT); the
+ * handle's fields are not touched and its next loops run as ever.  WF_ERR_UNSUPPORTED where
+ * the loop has no split of several blocks. */
+int wf_loop_wait_selftest(wf_solver* h, int kernel, int silent_block, int rounds, int* status);
 /* Which kernels run the Jacobi loops (no counterpart in the reference).
  * WF_LOOPS_AUTO (default): a loop whose grid fits the GPU's registers and
  * shared memories runs as one cooperative launch that keeps it there, any

@@ -202,6 +202,7 @@ _SIGNATURES = {
     "wf_get_tiles": (c_int, [c_void_p, POINTER(c_int), POINTER(c_int), POINTER(c_int), POINTER(c_int)]),
     "wf_set_blocking": (c_int, [c_void_p, c_int, c_int]),
     "wf_set_loops": (c_int, [c_void_p, c_int]),
+    "wf_loop_wait_selftest": (c_int, [c_void_p, c_int, c_int, c_int, POINTER(c_int)]),
     "wf_get_loop_plan": (c_int, [c_void_p, c_int, c_int, POINTER(c_int), POINTER(c_int), POINTER(c_int)]),
     "wf_get_blocking": (c_int, [c_void_p, POINTER(c_int), POINTER(c_int)]),
     "wf_export_open": (c_int, [c_void_p, c_char_p, c_int, c_int, c_int, POINTER(c_void_p)]),

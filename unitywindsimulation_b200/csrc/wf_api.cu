@@ -1472,6 +1472,42 @@ int wf_stage_wait_selftest(wf_solver* h, int short_stage, double timeout_ms, int
     return WF_OK;
 }
 
+int wf_loop_wait_selftest(wf_solver* h, int kernel, int silent_block, int rounds, int* status) {
+    if (!h) return WF_ERR_INVALID_ARG;
+    const bool vel = kernel == WF_KERNEL_VEL_SWEEP;
+    const wf::ResPlan& pl = vel ? h->res.vel : h->nonuniform ? h->res.nupres_alone() : h->res.pres_alone();
+    if (!status || rounds < 1 || rounds > wf::kWaitRounds || (!vel && kernel != WF_KERNEL_PRES_SWEEP))
+        return set_err(h, WF_ERR_INVALID_ARG, "bad kernel id, rounds or status pointer");
+    if (!wf::loops_on_chip(h, pl) || pl.boxes() < 2)
+        return set_err(h, WF_ERR_UNSUPPORTED, "the loop has no split of several blocks");
+    if (silent_block < -1 || silent_block >= pl.boxes()) return set_err(h, WF_ERR_INVALID_ARG, "no such block");
+    WF_CUDA(cudaSetDevice(h->device));
+    WF_TRY(sync(h));
+    const size_t N = h->P.N;
+    float* it = nullptr;
+    if (cudaMalloc(&it, 6 * N * sizeof(float)) != cudaSuccess) {
+        cudaGetLastError();
+        return set_err(h, WF_ERR_OOM, "scratch iterates");
+    }
+    wf::ResWork w = h->res.work;  // the handle's own packets: later loops use the same slots
+    w.rounds = rounds;
+    w.silent = silent_block;
+    const int n = 5;
+    cudaError_t e = cudaMemsetAsync(it, 0, 6 * N * sizeof(float), h->st);
+    if (e == cudaSuccess && vel)
+        e = wf::launch_res_vel(h->P, h->st, pl, w, h->vcoef, h->vcoef + 6 * N, h->bv, it, it + 3 * N, nullptr, n, h->dstat);
+    else if (e == cudaSuccess && h->nonuniform)
+        e = wf::launch_res_nupres(h->P, h->st, pl, w, h->nucoef, h->bp, it, it + N, it + 2 * N, n, h->dstat);
+    else if (e == cudaSuccess)
+        e = wf::launch_res_pres(h->P, h->st, pl, w, h->pcoef, h->pcoef + 3 * N, h->bp, it, it + N, it + 2 * N, nullptr, n,
+                                h->dstat);
+    const int s = e == cudaSuccess ? sync(h) : WF_ERR_CUDA;
+    cudaFree(it);
+    if (s != WF_OK && s != WF_ERR_TIMEOUT) return set_err(h, s, "the loop did not run");
+    *status = s;
+    return WF_OK;
+}
+
 int wf_time_kernel(wf_solver* h, int kernel, int reps, int flush_l2, float* ms_per_launch,
                    double* alg_bytes_per_launch, int* sweeps_per_launch) {
     if (!h) return WF_ERR_INVALID_ARG;

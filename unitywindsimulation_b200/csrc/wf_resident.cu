@@ -32,7 +32,7 @@
 //
 // The launch is cooperative, so all blocks are resident and every packet
 // that is waited for will be sent.  The waits are bounded all the same
-// (kRounds): a wait that runs out sets *status and the block returns, its
+// (kWaitRounds): a wait that runs out sets *status and the block returns, its
 // neighbours' waits then run out as well.
 #include <cuda_runtime.h>
 
@@ -46,9 +46,6 @@ namespace wf {
 namespace {
 
 constexpr int NT = 512;                               // threads of a block, one z column each
-// Limit of one wait, in polling rounds: a round is one trip to L2 (0.2 to
-// 0.5 us), so a wait ends after one to two seconds.
-constexpr int kRounds = 1 << 22;
 constexpr int kMaxBoxes = 256;
 constexpr size_t kSmemMax = 232448 - 1024;
 
@@ -229,14 +226,14 @@ __device__ __forceinline__ Links make_links(const Box& b, const ResPlan& pl, boo
 // False where the rounds ran out.
 template <int R, bool RIM>
 __device__ __forceinline__ bool receive(const Links& l, int rim, float* v, const unsigned long long* pk, unsigned ep,
-                                        float& hu, float& hd) {
+                                        int rounds, float& hu, float& hd) {
     const bool nu = l.ru >= 0, nd = l.rd >= 0, ne = RIM && l.re >= 0;
     const unsigned long long *pu = pk + (nu ? l.ru : 0), *pd = pk + (nd ? l.rd : 0), *pe = pk + (ne ? l.re : 0);
     constexpr int U = !RIM ? 0 : R <= 8 ? R : (R + 1) / 2;
 #pragma unroll
     for (int r0 = 0; r0 < (RIM ? R : 1); r0 += RIM ? U : 1) {
         unsigned long long w[U + 1], wu = 0, wd = 0;
-        int left = kRounds;
+        int left = rounds;
         bool ok;
         do {
             if (r0 == 0) {
@@ -296,6 +293,7 @@ struct PresArgs {
     size_t half;                   // packets of one parity
     unsigned* ctl;
     int* status;
+    int rounds, silent;            // limit of a wait; block that sends nothing
 };
 
 // The loops read every neighbour, fluid or not, through a coefficient that is 0 on
@@ -363,7 +361,8 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
     const bool inxy = own && x < a.nx && y < a.ny;
     const int i0 = inxy ? (b.z0 * a.ny + y) * a.nx + x : 0;
     const int o0 = (ly + 1) * b.sx + lx + 1;
-    const Links l = make_links(b, a.pl, own, 1);
+    Links l = make_links(b, a.pl, own, 1);
+    if (b.id == a.silent) l.se = l.su = l.sd = -1;
     // the input iterate with its halo, zero outside the domain
     for (int o = tid; o < 2 * R * PS; o += NT) sm[o] = 0.f;
     __syncthreads();
@@ -492,8 +491,8 @@ __global__ void __launch_bounds__(NT, 1) k_res_pres(const __grid_constant__ Pres
         }
         if (STACK) keep(k);
         if (has_halo)
-            bad = rim ? !receive<R, true>(l, b.rim, nxt - o0, pk, ep, hu, hd)
-                      : !receive<R, false>(l, b.rim, nxt - o0, pk, ep, hu, hd);
+            bad = rim ? !receive<R, true>(l, b.rim, nxt - o0, pk, ep, a.rounds, hu, hd)
+                      : !receive<R, false>(l, b.rim, nxt - o0, pk, ep, a.rounds, hu, hd);
         if (__syncthreads_or(bad)) break;
         float* t = cur;
         cur = nxt;
@@ -639,7 +638,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_pair(const __grid_constant__ Pres
     const int oE = col && lx == bx ? w * (by + 4) + by + ly : o + 1, oW = col && lx < 0 ? w * (by + 4) + ly : o - 1;
     const int i0 = col ? y * a.nx + x : 0;
     const int slot = id * cells + ly * bx + lx;
-    const bool edge = own && (lx < 2 || lx >= bx - 2 || ly < 2 || ly >= by - 2);
+    const bool sends = H > 0 && id != a.silent;  // every cell: with 4 cells a thread at most few are not read
     const bool mine = own && col, lo = mine && z0 > 0, hi = mine && z0 + R < a.nz;
     // coefficients of the column's cells, j = 0 .. R + 1 for z = -1 .. R
     float cE[E], cW[E], cN[E], cS[E], cU[E], cD[NU ? E : 1], ai[E], rh[E];
@@ -716,12 +715,12 @@ __global__ void __launch_bounds__(NT, 1) k_res_pair(const __grid_constant__ Pres
             unsigned long long* dst = pk + slot;
 #pragma unroll
             for (int j = 1; j <= R; ++j)
-                if (H > 0 && (R <= 4 || edge || j <= 2 || j >= R - 1)) put(dst + (j - 1) * bx * by, v[j], ep);
+                if (sends) put(dst + (j - 1) * bx * by, v[j], ep);
 #pragma unroll
             for (int j = 1; j <= R; ++j)
                 if (keep >> j & 1u) s0[o + (j + 1) * PS] = v[j];
         }
-        int left = kRounds;
+        int left = a.rounds;
         if (H > 0) {
             const long long t0 = clock64();
             while (clock64() - t0 < kPairWait) {}
@@ -797,6 +796,7 @@ struct VelArgs {
     size_t half;
     unsigned* ctl;
     int* status;
+    int rounds, silent;
     float* stream;   // k_res_vel_wide: the words read in every sweep
     float* stack;    // iterate k of every cell goes to stack + k step
     long long step;
@@ -812,14 +812,14 @@ struct VelArgs {
 // 48 1.58 / 1.38 / 1.30, 72 x 40 x 72 - / 1.61 / 1.55, 100 x 50 x 100 3.72 / 3.38 /
 // 2.96.
 template <int F, int CS>
-__device__ __forceinline__ bool receive3(const Links& l, float* v, const Packet3* pk, unsigned ep, float hu[3],
-                                         float hd[3]) {
+__device__ __forceinline__ bool receive3(const Links& l, float* v, const Packet3* pk, unsigned ep, int rounds,
+                                         float hu[3], float hd[3]) {
     const bool nu = l.ru >= 0, nd = l.rd >= 0;
     const Packet3 *pu = pk + (nu ? l.ru : 0), *pd = pk + (nd ? l.rd : 0);
     // (the exception saves registers where F is 4: 6.97 -> 6.67 us on 149 x 61 x 103)
     auto need = [&](int q) { return l.re >= 0 && ((F > 3 && q == 0) || q < l.rn); };
     Packet3 w[F], wu, wd;
-    int left = kRounds;
+    int left = rounds;
     bool ok;
     do {
         wu = get3(pu);
@@ -867,7 +867,8 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
     const bool inxy = own && x < a.nx && y < a.ny;
     const int i0 = inxy ? (b.z0 * a.ny + y) * a.nx + x : 0;
     const int o0 = (ly + 1) * b.sx + lx + 1;
-    const Links l = make_links(b, a.pl, own, NT / (b.rim + 4));
+    Links l = make_links(b, a.pl, own, NT / (b.rim + 4));
+    if (b.id == a.silent) l.se = l.su = l.sd = -1;
     // the input iterate with its halo, zero outside the domain
     for (int o = tid; o < 3 * CS; o += NT) sm[o] = 0.f;
     __syncthreads();
@@ -1007,7 +1008,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel(const __grid_constant__ VelAr
                 for (int r = 0; r < R; ++r) cur[c * CS + r * PS] = u[c][r];
         }
         if (STACK) keep(k);
-        if (gridDim.x > 1) bad = !receive3<fetch_max(R), CS>(l, sm, pk, ep, hu, hd);
+        if (gridDim.x > 1) bad = !receive3<fetch_max(R), CS>(l, sm, pk, ep, a.rounds, hu, hd);
         if (__syncthreads_or(bad)) break;
         Packet3* t = pk;
         pk = pk_next;
@@ -1123,6 +1124,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel_wide(const __grid_constant__ 
                 l.rd = (b.id - layer) * b.slots + top + tid;
             }
         }
+        if (b.id == a.silent) l.se = l.su = l.sd = -1;
     }
     const int g = tid / (b.rim + 4), e = tid % (b.rim + 4);
     int ht, hx, hy;
@@ -1244,7 +1246,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_vel_wide(const __grid_constant__ 
             if (r == R - 1 && l.su >= 0) put3(pk + l.su, v[0], v[1], v[2], ep);
         });
         fetch(R - 1);
-        if (gridDim.x > 1) bad = !receive3<(R + kGroup - 1) / kGroup, CS>(l, nb, pk, ep, hu, hd);
+        if (gridDim.x > 1) bad = !receive3<(R + kGroup - 1) / kGroup, CS>(l, nb, pk, ep, a.rounds, hu, hd);
         if (__syncthreads_or(bad)) break;
         Packet3* t = pk;
         pk = pk_next;
@@ -1502,6 +1504,8 @@ cudaError_t launch_pres(PresKernel k, const Params& P, cudaStream_t st, const Re
     a.half = packets(pl);
     a.ctl = w.ctl;
     a.status = status;
+    a.rounds = w.rounds;
+    a.silent = w.silent;
     const cudaError_t e = launch_coop((const void*)k, pl.boxes(), pl.pair ? pair_smem(pl) : pres_smem(pl.bz), st, &a);
     if (e == cudaSuccess) WF_COUNT_LAUNCH();
     else cudaGetLastError();
@@ -1538,6 +1542,8 @@ cudaError_t launch_res_vel(const Params& P, cudaStream_t st, const ResPlan& pl, 
     a.half = packets(pl);
     a.ctl = w.ctl;
     a.status = status;
+    a.rounds = w.rounds;
+    a.silent = w.silent;
     a.stream = w.stream;
     a.stack = stack;
     a.step = step;

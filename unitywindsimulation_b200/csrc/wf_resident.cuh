@@ -18,11 +18,16 @@ struct ResPlan {
 
 // Device workspace of the loops of one stream: the halo packets of both
 // parities, the epoch words and streamed coefficients.  One loop at a time may use it.
+// Limit of one wait, in polling rounds: a round is one trip to L2 (0.2 to
+// 0.5 us), so a wait ends after one to two seconds.
+constexpr int kWaitRounds = 1 << 22;
 struct ResWork {
     void* pk = nullptr;    // the allocation; 64-bit packets of the pressure loops
     void* pk3 = nullptr;   // 128-bit packets of the momentum loop
     unsigned* ctl = nullptr;
     float* stream = nullptr;  // coefficients the momentum loop reads in every sweep
+    int rounds = kWaitRounds;
+    int silent = -1;          // block that sends nothing (the self-test of the waits)
 };
 
 // The plans of one handle's loops and their workspace.
