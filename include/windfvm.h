@@ -484,7 +484,9 @@ int wf_loop_wait_selftest(wf_solver* h, int kernel, int silent_block, int rounds
  * shared memories runs as one cooperative launch that keeps it there, any
  * other as passes over memory.  WF_LOOPS_PASSES: passes always; an explicit
  * depth or tile (wf_set_blocking, wf_set_tiles) selects it too.  Results do
- * not depend on the mode.  Drops the handle's captured step graphs; rebuild
+ * not depend on the mode, but for what is not finite: a pass of several pressure
+ * sweeps carries the NaN of a fluid cell without fluid neighbours through walls of up to
+ * three cells, a loop on chip and one sweep a launch keep it in its cell.  Drops the handle's captured step graphs; rebuild
  * batches that contain the handle afterwards. */
 enum { WF_LOOPS_AUTO = 0, WF_LOOPS_PASSES = 1 };
 int wf_set_loops(wf_solver* h, int mode);

@@ -912,16 +912,16 @@ int adj_fail(wf_adjoint* a, int code, const char* msg) {
         }                                                                      \
     } while (0)
 
-// WF_ERR_TIMEOUT when a bounded wait of the TMA-staged pressure passes ran
-// out since the last check (the solver's sticky wait status).
+// WF_ERR_TIMEOUT when a bounded wait of the TMA-staged pressure passes or of a
+// loop on chip ran out since the last check (the solver's sticky wait status).
 int adj_check_waits(wf_adjoint* a) {
     volatile int* st = a->h->hstat;
     if (!st || !*st) return WF_OK;
     *st = 0;
-    return adj_fail(a, WF_ERR_TIMEOUT, "a bounded wait of a pressure loop's kernel ran out; results are not valid");
+    return adj_fail(a, WF_ERR_TIMEOUT, "a bounded wait of a Jacobi loop's kernel ran out; results are not valid");
 }
 
-// On-chip pressure loops, or nullptr where the solver runs the pass kernels.
+// Loops on chip, or nullptr where the solver runs the pass kernels.
 const wf::Resident* adj_resident(const wf_adjoint* a) { return a->h->resident && a->h->dstat ? &a->res : nullptr; }
 // n momentum sweeps from u^0 on chip with every iterate kept (u^k at u0 + k step);
 // the transposed sweeps are the forward ones with A^T and no right-hand side.  One

@@ -299,7 +299,8 @@ int do_pres_sweeps(wf_solver* h, int n, bool allow_fast) {
     // with residual checks: the sweeps up to the next one on chip, in the
     // sums of the kernels below.  One sweep a launch took 6.5 of the 8.2 ms of
     // a step on 100 x 50 x 100 (400 sweeps, checked every 20).  (The momentum
-    // loop has no such form: 12 instead of 7 coefficients a cell do not fit.)
+    // loop has none in the sums of its kernel below, which keeps convection and diffusion
+    // apart: 12 words a cell instead of 6 with a turbulence model, 6 without; not built.)
     const bool chip = allow_fast && resid && wf::loops_on_chip(h, h->nonuniform ? h->res.nupres_alone() : h->res.pres_alone());
     bool coef_done = false;
     for (int k = 0; k < n; ++k) {

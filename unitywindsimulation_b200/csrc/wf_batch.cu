@@ -587,7 +587,7 @@ int wf_batch_step(wf_batch* b, int n_steps) {
             waits_ran_out = true;
         }
     if (waits_ran_out)
-        return fail(b, WF_ERR_TIMEOUT, "a bounded wait of a TMA-staged pressure pass ran out; the cases' fields are "
+        return fail(b, WF_ERR_TIMEOUT, "a bounded wait of a Jacobi loop's kernel ran out; the cases' fields are "
                                        "not valid");
     if (persistent) {
         wf::GridBar hb{};

@@ -530,7 +530,7 @@ __global__ void k_vel_precompute(const __grid_constant__ Params P, const Bnd B, 
 // of the same D.
 // Bound by the latency of its 41 loads; all of them leave before the first use,
 // with the neighbour mask for six flag reads and the reciprocals for three
-// divisions: 20.5 -> 11.0 us a sweep on 100 x 50 x 100.
+// divisions: 20.5 -> 12.5 us a sweep on 100 x 50 x 100 (ncu, cold).
 __global__ void k_vel_sweep(const __grid_constant__ Params P, const float* __restrict__ uI,
                             const float* __restrict__ uT, const float* __restrict__ eddy,
                             const float* __restrict__ Dv, const float* __restrict__ iD,

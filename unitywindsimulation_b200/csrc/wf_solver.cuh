@@ -95,7 +95,7 @@ struct wf_solver {
     int pres_ty = 32;         // tile rows of the pressure multi-sweep kernel (32 or 16)
     int pres_tma = 1;         // four-sweep passes with TMA-staged tiles where they apply
                               // (WF_TMA=0: the per-thread-staged kernel; same iterates)
-    // sticky status of the bounded waits in the TMA-staged kernel: page-locked
+    // sticky status of the bounded waits in the TMA-staged kernels and the loops on chip: page-locked
     // host word (hstat) and its device alias (dstat); nonzero = a wait ran out
     int* hstat = nullptr;
     int* dstat = nullptr;
