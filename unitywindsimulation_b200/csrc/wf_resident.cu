@@ -20,15 +20,11 @@
 //
 // What bounds it: the trip of the packets (470 cycles within a die, 900 across,
 // measured SM to SM) and the instructions of a column, one warp after another;
-// not memory.  Measured, us a pressure sweep: 0.77 on 64 x 32 x 48 and 0.81 on 80 x
-// 40 x 40 (two sweeps a trip, k_res_pair; 1.10 and 1.16 with one), 1.74 on 100 x 50 x
-// 100, 2.3 on 128 x 64 x 96, 3.5 on 149 x 61 x 103; a momentum sweep: 1.30, 1.41,
-// 2.96, 4.7 and 6.6.  Whole steps, with one launch for every one to four sweeps
-// before: 623 -> 234 us (64 x 32 x 48, PISO, 50 momentum and 90 pressure sweeps),
-// 5077 -> 1026 us (80 x 40 x 40, 100 and 1000), 2429 -> 944 us (100 x 50 x 100, 50 and
-// 400), 1279 -> 977 us (128 x 64 x 96, 50 and 90, its fields read back), 1397 -> 970 us
-// (149 x 61 x 103, 50 and 90), 9759 -> 6226 us (100 x 50 x 100 stretched mesh, 800 and
-// 2000).
+// not memory.  Measured, us a pressure sweep: 0.75 on 64 x 32 x 48 and 0.80 on 80 x
+// 40 x 40 (two sweeps a trip, k_res_pair; 1.10 and 1.16 with one), 1.69 on 100 x 50 x
+// 100, 2.3 on 128 x 64 x 96, 3.6 on 149 x 61 x 103; a momentum sweep: 1.35, 1.44,
+// 2.9, 4.7 and 6.7.  With one launch for every one to four sweeps: 4.7, 4.7, 5.2, 5.2,
+// 6.3 and 2.1, 3.0, 5.6, 6.1, 11.6.
 //
 // The launch is cooperative, so all blocks are resident and every packet
 // that is waited for will be sent.  The waits are bounded all the same

@@ -171,8 +171,8 @@ inline bool shares(const wf_solver* h, const ResPlan& p) { return p.bz > 0 && 2 
 // least half of them to the others.  A larger case keeps its pressure split for
 // a lone case and its momentum passes.  Us a batched step: 16 cases of 0.06-0.21 M
 // cells 3370 in passes, 3770 with lone splits (one loop after another), 2061
-// with shared ones (1950 now); 16 cases of 0.7-1.75 M cells 20600 in passes, 19600
-// with this rule (18480 now), 28800 with shared splits whatever their size and 27900
+// with shared ones (1920 now); 16 cases of 0.7-1.75 M cells 20600 in passes, 19600
+// with this rule (18500 now), 28800 with shared splits whatever their size and 27900
 // with lone momentum splits too (loops of more than half the GPU each wait for it
 // to empty).
 inline const ResPlan& pres_plan(const wf_solver* h) {
