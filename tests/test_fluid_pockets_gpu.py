@@ -35,11 +35,11 @@ def _faces(n):
 def _case(grid, kind):
     nx, ny, nz = grid
     if kind == "stretched":
-        case = cases.small_nonuniform_case(nv=5, np_=19)
+        case = cases.small_nonuniform_case(nv=24, np_=19)
         case.cfg.nx, case.cfg.ny, case.cfg.nz = grid
         case.faces = tuple(_faces(n) for n in grid)
     else:
-        case = cases.small_case(nx=nx, ny=ny, nz=nz, seed=1, nv=5, np_=19, piso=kind == "piso")
+        case = cases.small_case(nx=nx, ny=ny, nz=nz, seed=1, nv=24, np_=19, piso=kind == "piso")
     if kind == "checked":
         case.cfg.calc_residual, case.cfg.vel_res_interval, case.cfg.pres_res_interval = 1, 4, 9
         case.cfg.vel_tol = case.cfg.pres_tol = 1e-30

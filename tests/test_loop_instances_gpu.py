@@ -79,14 +79,14 @@ def _same(a, b):
 
 @pytest.mark.parametrize("grid", GRIDS, ids=ids)
 def test_steps(built, grid):
-    a, b = _pair(_case(grid, nv=6, np_=9, les=grid[2] % 2 == 0, piso=grid[1] % 2 == 0))
+    a, b = _pair(_case(grid, nv=20, np_=20, les=grid[2] % 2 == 0, piso=grid[1] % 2 == 0))
     _step(a, b, 2)
     _same(a, b)
 
 
 @pytest.mark.parametrize("grid", GRIDS, ids=ids)
 def test_checked_steps(built, grid):
-    case = _case(grid, nv=5, np_=14, piso=False)
+    case = _case(grid, nv=5, np_=20, piso=False)
     case.cfg.calc_residual, case.cfg.vel_res_interval, case.cfg.pres_res_interval = 1, 4, 5
     case.cfg.vel_tol = case.cfg.pres_tol = 1e-30
     a, b = _pair(case, momentum=False)
@@ -97,17 +97,17 @@ def test_checked_steps(built, grid):
 
 @pytest.mark.parametrize("grid", STRETCHED, ids=ids)
 def test_stretched_steps(built, grid):
-    a, b = _pair(_case(grid, stretched=True, nv=6, np_=9, log_inflow=grid[2] % 2 == 0))
+    a, b = _pair(_case(grid, stretched=True, nv=20, np_=20, log_inflow=grid[2] % 2 == 0))
     _step(a, b, 2)
-    a.op("pres_sweeps", 4)
-    b.op("pres_sweeps", 4)
+    a.op("pres_sweeps", 17)
+    b.op("pres_sweeps", 17)
     _same(a, b)
     assert np.array_equal(a.get_face_flux(), b.get_face_flux())
 
 
 @pytest.mark.parametrize("grid", STRETCHED, ids=ids)
 def test_stretched_checked_steps(built, grid):
-    case = _case(grid, stretched=True, nv=5, np_=14)
+    case = _case(grid, stretched=True, nv=5, np_=20)
     case.cfg.calc_residual, case.cfg.vel_res_interval, case.cfg.pres_res_interval = 1, 4, 5
     case.cfg.vel_tol = case.cfg.pres_tol = 1e-30
     a, b = _pair(case, momentum=False)
@@ -119,11 +119,11 @@ def test_stretched_checked_steps(built, grid):
 @pytest.mark.parametrize("grid", GRIDS, ids=ids)
 def test_last_iterates(built, grid):
     """Outside a step the loops also leave iterate n - 1, and start from the last one."""
-    a, b = _pair(_case(grid, nv=4, np_=4))
+    a, b = _pair(_case(grid, nv=20, np_=20))
     for s in (a, b):
         s.Step(1)
-        s.op("vel_precompute"); s.op("vel_sweeps", 3); s.op("vel_sweeps", 2); s.op("pres_precompute")
-        for n in (2, 3, 5):
+        s.op("vel_precompute"); s.op("vel_sweeps", 20); s.op("vel_sweeps", 21); s.op("pres_precompute")
+        for n in (5, 6, 9):
             s.op("pres_sweeps", n)
     _same(a, b)
 
@@ -132,7 +132,7 @@ def test_last_iterates(built, grid):
 def test_adjoint_iterates(built, grid):
     """The kept iterates with 4 and 8 cells a thread: the recorded step bit for bit, the
     reversed one to the rounding of its float atomics."""
-    case = cases.small_soft_case(*grid, nv=5, np_=6)
+    case = cases.small_soft_case(*grid, nv=20, np_=20)
     rng = np.random.default_rng(1)
     n = case.n_cells
     ub, pb = rng.standard_normal((3, n), dtype=np.float32), rng.standard_normal(n, dtype=np.float32)
@@ -154,7 +154,7 @@ def test_batches(built, grid):
     from unitywindsimulation_b200.solver import BatchSolver
     alone, batched, passes = ([], [], [])
     for seed in (0, 1):
-        case = cases.small_case(nx=grid[0], ny=grid[1], nz=grid[2], seed=seed, nv=6, np_=9)
+        case = cases.small_case(nx=grid[0], ny=grid[1], nz=grid[2], seed=seed, nv=20, np_=20)
         for group, mode in ((alone, _lib.LOOPS_AUTO), (batched, _lib.LOOPS_AUTO), (passes, _lib.LOOPS_PASSES)):
             s = FvmSolverCuda(case.cfg)
             s.set_loops(mode)

@@ -21,14 +21,14 @@ def _faces(n):
 def _solver(grid, stretched):
     nx, ny, nz = grid
     if stretched:
-        case = cases.small_nonuniform_case(nv=6, np_=9)
+        case = cases.small_nonuniform_case(nv=20, np_=20)
         box = case.flags
         case.cfg.nx, case.cfg.ny, case.cfg.nz = grid
         case.faces = tuple(_faces(n) for n in grid)
         case.flags = np.zeros((nz, ny, nx), np.int32)
         case.flags[:box.shape[0], :box.shape[1], :box.shape[2]] = box
     else:
-        case = cases.small_case(nx=nx, ny=ny, nz=nz, seed=4, nv=6, np_=9)
+        case = cases.small_case(nx=nx, ny=ny, nz=nz, seed=4, nv=20, np_=20)
     s = FvmSolverCuda(case.cfg)
     cases.apply_case(s, case)
     s.Step(2)

@@ -78,7 +78,7 @@ def test_fields_do_not_depend_on_company(built, stretched):
     """Round robin, one thread a handle, and with readbacks instead of waits, against
     stepping one after another."""
     grids = [g for g in GRIDS if not stretched or min(g) >= 10]
-    cs = [_case(g, stretched, i, nv=7, np_=23) for i, g in enumerate(grids)]
+    cs = [_case(g, stretched, i, nv=20, np_=23) for i, g in enumerate(grids)]
     alone, beside = _handles(cs), _handles(cs)
     for s in alone:
         s.Step(15)

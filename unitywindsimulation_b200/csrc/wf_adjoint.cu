@@ -930,7 +930,7 @@ const wf::Resident* adj_resident(const wf_adjoint* a) { return a->h->resident &&
 // sweeps.
 bool vel_on_chip(wf_adjoint* a, const float* A, const float* iD, const float* b, float* u0, int n, long long step) {
     const wf::Resident* r = adj_resident(a);
-    return r && n >= 2 && r->ok(r->vel) &&
+    return r && n >= r->vel.least && r->ok(r->vel) &&
            wf::launch_res_vel(a->h->P, a->st, r->vel, r->work, A, iD, b, u0, nullptr, nullptr, n, a->h->dstat, u0,
                               step) == cudaSuccess;
 }

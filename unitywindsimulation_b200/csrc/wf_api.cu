@@ -12,6 +12,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -293,7 +294,7 @@ int do_pres_sweeps(wf_solver* h, int n, bool allow_fast) {
         WF_TRY(wf::pres_sweeps_fast(h, n, /*piso=*/false));
         return WF_OK;
     }
-    if (allow_fast && !resid && n >= 2 && wf::loops_on_chip(h, wf::nupres_plan(h)) &&
+    if (allow_fast && !resid && wf::loops_on_chip(h, wf::nupres_plan(h), n) &&
         wf::pres_sweeps_on_chip(h, n, true, !h->in_step))
         return WF_OK;
     // with residual checks: the sweeps up to the next one on chip, in the
@@ -301,7 +302,9 @@ int do_pres_sweeps(wf_solver* h, int n, bool allow_fast) {
     // a step on 100 x 50 x 100 (400 sweeps, checked every 20).  (The momentum
     // loop has none in the sums of its kernel below, which keeps convection and diffusion
     // apart: 12 words a cell instead of 6 with a turbulence model, 6 without; not built.)
-    const bool chip = allow_fast && resid && wf::loops_on_chip(h, h->nonuniform ? h->res.nupres_alone() : h->res.pres_alone());
+    const wf::ResPlan& plan = h->nonuniform ? h->res.nupres_alone() : h->res.pres_alone();
+    const int least = wf::least_between_checks(h);
+    const bool chip = allow_fast && resid && wf::loops_on_chip(h, plan, INT_MAX);
     bool coef_done = false;
     for (int k = 0; k < n; ++k) {
         const float* src = h->pc_zero ? nullptr : h->pcb[h->iPCL];
@@ -319,7 +322,7 @@ int do_pres_sweeps(wf_solver* h, int n, bool allow_fast) {
         const int interval = h->cfg.pres_res_interval;
         for (;;) {
             const int m = std::min((k / interval + 1) * interval, n - 1) - k;  // sweeps up to the next check
-            if (m < 2 || !wf::pres_sweeps_on_chip(h, m, coef_done, true)) break;
+            if (m < least || !wf::pres_sweeps_on_chip(h, m, coef_done, true)) break;
             coef_done = true;
             k += m;
             if (k % interval == 0) WF_TRY(pres_converged(h, h->pcb[h->iPC], h->pcb[h->iPCL], &done));
@@ -1479,7 +1482,7 @@ int wf_loop_wait_selftest(wf_solver* h, int kernel, int silent_block, int rounds
     const wf::ResPlan& pl = vel ? h->res.vel : h->nonuniform ? h->res.nupres_alone() : h->res.pres_alone();
     if (!status || rounds < 1 || rounds > wf::kWaitRounds || (!vel && kernel != WF_KERNEL_PRES_SWEEP))
         return set_err(h, WF_ERR_INVALID_ARG, "bad kernel id, rounds or status pointer");
-    if (!wf::loops_on_chip(h, pl) || pl.boxes() < 2)
+    if (!wf::loops_on_chip(h, pl, INT_MAX) || pl.boxes() < 2)
         return set_err(h, WF_ERR_UNSUPPORTED, "the loop has no split of several blocks");
     if (silent_block < -1 || silent_block >= pl.boxes()) return set_err(h, WF_ERR_INVALID_ARG, "no such block");
     WF_CUDA(cudaSetDevice(h->device));

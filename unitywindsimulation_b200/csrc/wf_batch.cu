@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <map>
 #include <string>
@@ -759,7 +760,8 @@ int wf_get_loop_plan(const wf_solver* h, int kernel, int beside, int* blocks, in
     // the pressure sweeps from check to check after the first
     const int n = vel ? c.calc_residual ? 1 : c.vel_iters
                       : c.calc_residual ? std::min(c.pres_res_interval, c.pres_iters - 1) : c.pres_iters;
-    const bool chip = h->fast && n >= 2 && wf::loops_on_chip(h, p);
+    const int least = !vel && c.calc_residual ? wf::least_between_checks(h) : p.least;
+    const bool chip = h->fast && n >= least && wf::loops_on_chip(h, p, INT_MAX);
     *blocks = chip ? p.boxes() : 0;
     *cells = chip ? p.bz : 0;
     *sweeps_per_trip = !chip ? 0 : p.pair ? 2 : 1;

@@ -33,6 +33,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <iterator>
 
 #include "wf_kernels.cuh"
@@ -1374,6 +1375,40 @@ ResPlan make_plan(const Params& P, int sms, const int (&Rs)[M], Loop loop = Loop
     }
     return best;
 }
+// A loop on chip first reads its coefficients, every box at once: 5 us with 2 cells a
+// thread, 20 to 40 with 8 to 16, what a few sweeps in passes take.  The least number of
+// sweeps that pay for it, from the times of loops of 2 to 48 sweeps on 75 grids of 27 to
+// 1.1 M cells, cubes, sheets and needles.
+// Pressure, by cells a thread.  Uniform: four sweeps a pass take 19 us on any of these
+// grids, one or two little less; even at 1 to 2.6 sweeps with up to 8 cells a thread, 3 to 4.5
+// above (two sweeps on 149 x 61 x 103 +8 us, five -1).  Stretched: a sweep in passes takes
+// 1.2 to 2.4 us; even at 5 to 9 sweeps with 2 and 3 cells a thread, 5 to 12 with 4 and 6, 15
+// with 8 (100 x 50 x 100: 8 sweeps +6 us, 24 -6).
+int least_pres(const ResPlan& p, bool stretched) {
+    const int R = p.bz;
+    if (stretched) return R <= 3 ? 9 : R <= 6 ? 12 : 16;
+    return R <= 6 ? 2 : R <= 8 ? 3 : R <= 12 ? 4 : 5;
+}
+// Momentum: the start and a sweep's time by cells a thread (a sweep of boxes with few
+// columns takes less), against a sweep in passes: four cells a thread 1.8 us up to 0.1 M
+// cells, 5.1 at 0.5 M, 6.3 at 0.86 M; one cell a thread (nx % 4 != 0) 2.4 + 9.3 a million.  Even
+// (computed, measured): 64 x 32 x 48 15, 11; 72 x 40 x 72 8, 5; 100 x 50 x 100 11, 9; 128 x 64
+// x 96 21, 20; 149 x 61 x 103 10, 8; 128 x 60 x 112 and needles such as 3 x 3 x 2000 never.
+int least_vel(const Params& P, const ResPlan& p) {
+    static constexpr struct { int R; double start, sweep; } kCost[] = {
+        {2, 7, 1.40}, {3, 8.7, 1.45}, {4, 9.7, 1.55}, {6, 14, 2.2}, {8, 22, 2.95},
+        {10, 20, 3.95}, {12, 26, 4.7}, {14, 35, 6.2}, {15, 39, 6.8}};
+    const double m = 1e-6 * P.N, fill = (double)P.N / ((double)p.boxes() * NT * p.bz);
+    const double pass = P.nx % 4 == 0 ? std::max(1.8, m < 0.5 ? 1.8 + 8.25 * (m - 0.1) : 5.1 + 3.3 * (m - 0.5))
+                                      : 2.35 + 9.3 * m;
+    for (const auto& c : kCost) {
+        if (c.R != p.bz) continue;
+        const double thin = 0.6 + 0.18 * c.R;
+        const double gain = pass - (thin + (c.sweep - thin) * std::min(1.0, fill / 0.75));
+        return gain > 0.0 ? std::max(2, (int)std::min(c.start / gain + 1.0, 1e9)) : INT_MAX;
+    }
+    return 2;
+}
 // Words of the momentum loop's streamed coefficients.
 size_t streamed(const ResPlan& p) {
     return p.bz > kVelR[std::size(kVelR) - 1] ? (size_t)p.boxes() * p.bz * wide_streamed(p.bz) * NT : 0;
@@ -1445,6 +1480,9 @@ void resident_plan(const Params& P, int sms, Resident* r) {
     r->nupres2 = r->pres2;
     r->vel = make_plan(P, sms, kVelR, Loop::kVel);
     if (r->vel.bz == 0) r->vel = make_plan(P, sms, kVelWideR, Loop::kVelWide);
+    for (ResPlan* p : {&r->pres, &r->pres2}) p->least = least_pres(*p, false);
+    for (ResPlan* p : {&r->nupres, &r->nupres2}) p->least = least_pres(*p, true);
+    r->vel.least = least_vel(P, r->vel);
     r->pres_shared = make_plan(P, sms, kPresR, Loop::kPres, 1);
     r->vel_shared = make_plan(P, sms, kVelR, Loop::kVel, 1);
     // Beside other handles: an eighth of the multiprocessors costs nothing yet.
@@ -1454,6 +1492,13 @@ void resident_plan(const Params& P, int sms, Resident* r) {
     r->pres_beside = better(make_plan(P, sms, kPresR, Loop::kPres, part));
     r->nupres_beside = better(make_plan(P, sms, kNuPresR, Loop::kPres, part));
     r->vel_beside = make_plan(P, sms, kVelR, Loop::kVel, part);
+    // In company a loop counts by the multiprocessors it holds.  Steps of 2, 4 and 8 sweeps a
+    // loop, passes / chip: 16 cases of 24 x 12 x 16 in a batch 102 / 135, 141 / 155, 207 / 187 us, of
+    // 0.1 and 0.2 M cells 707 / 798, 874 / 886, 1199 / 1029; side by side 88 / 95, 128 / 101, 194
+    // / 117 and 726 / 798, 979 / 887, 1370 / 1017.
+    r->pres_shared.least = r->vel_shared.least = 6;
+    r->pres_beside.least = r->vel_beside.least = 4;
+    r->nupres_beside.least = least_pres(r->nupres_beside, true);
 }
 
 void resident_alloc(Resident* r, cudaStream_t st) {

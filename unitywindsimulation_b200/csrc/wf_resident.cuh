@@ -13,6 +13,7 @@ namespace wf {
 struct ResPlan {
     int bx = 0, by = 0, bz = 0, px = 0, py = 0, pz = 0;
     bool pair = false;   // pressure loop that runs two sweeps a halo trip
+    int least = 2;       // sweeps from which on the loop beats the passes
     int boxes() const { return px * py * pz; }
 };
 

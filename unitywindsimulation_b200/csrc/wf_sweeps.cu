@@ -918,7 +918,7 @@ int record_vel_loop(wf_solver* h, int n) {
 int vel_sweeps_fast(wf_solver* h, int n) {
     vel_coef(h);
     if (h->rec) return record_vel_loop(h, n);
-    if (n >= 2 && loops_on_chip(h, vel_plan(h))) {
+    if (loops_on_chip(h, vel_plan(h), n)) {
         // the whole loop on chip, into two buffers that are neither its input
         // nor velFieldLastTime
         const size_t N = h->P.N;
@@ -1096,7 +1096,7 @@ bool pres_sweeps_on_chip(wf_solver* h, int n, bool coef_done, bool keep_prev) {
 int pres_sweeps_fast(wf_solver* h, int n, bool piso) {
     const float* rhs = pres_coef(h, piso);
     if (h->rec) return record_pres_loop(h, n, rhs);
-    if (n >= 2 && loops_on_chip(h, pres_plan(h)) &&
+    if (loops_on_chip(h, pres_plan(h), n) &&
         pres_loop(h, !h->in_step, [&](const float* in, float* out, float* prev) {
             return launch_res_pres(h->P, h->st, pres_plan(h), h->res.work, h->pcoef, h->pcoef + 3 * (size_t)h->P.N, rhs,
                                    in, out, prev, nullptr, n, h->dstat);
@@ -1179,8 +1179,8 @@ int time_kernel(wf_solver* h, int which, int reps, bool flush, float* ms, double
     cudaEventCreate(&e1);
     float total = 0.f;
     // where the pressure loops run on chip one launch is a whole loop
-    const bool res_p = which == WF_KERNEL_PRES_SWEEP && loops_on_chip(h, pres_plan(h)) && h->cfg.pres_iters >= 2;
-    const bool res_v = which == WF_KERNEL_VEL_SWEEP && loops_on_chip(h, vel_plan(h)) && h->cfg.vel_iters >= 2;
+    const bool res_p = which == WF_KERNEL_PRES_SWEEP && loops_on_chip(h, pres_plan(h), h->cfg.pres_iters);
+    const bool res_v = which == WF_KERNEL_VEL_SWEEP && loops_on_chip(h, vel_plan(h), h->cfg.vel_iters);
     const int kv = res_v ? h->cfg.vel_iters : std::min(std::max(h->vel_k, 1), 2);
     const int kp = res_p ? h->cfg.pres_iters : std::min(std::max(h->pres_k, 1), 4);
     cudaError_t err = cudaSuccess;
@@ -1241,7 +1241,7 @@ void launch_stack_pass(const Params& P, cudaStream_t st, int sms, const float* c
 void launch_pres_stack(const Params& P, cudaStream_t st, int sms, const float* c3, const float* ainv,
                        const float* rhs, float* stack, int n, bool from_zero, int* status, const Resident* res) {
     const size_t N = P.N;
-    if (res && n >= 2 && res->ok(res->pres) &&
+    if (res && n >= res->pres.least && res->ok(res->pres) &&
         launch_res_pres(P, st, res->pres, res->work, c3, ainv, rhs, from_zero ? nullptr : stack, nullptr, nullptr,
                         stack, n, status) == cudaSuccess)
         return;
