@@ -481,8 +481,9 @@ int wf_set_blocking(wf_solver* h, int pres_k, int vel_k);
 int wf_loop_wait_selftest(wf_solver* h, int kernel, int silent_block, int rounds, int* status);
 /* Which kernels run the Jacobi loops (no counterpart in the reference).
  * WF_LOOPS_AUTO (default): a loop whose grid fits the GPU's registers and
- * shared memories runs as one cooperative launch that keeps it there, any
- * other as passes over memory.  WF_LOOPS_PASSES: passes always; an explicit
+ * shared memories runs as one cooperative launch that keeps it there, from
+ * the count of sweeps on that pays for its start; any other as passes over
+ * memory (wf_get_loop_plan).  WF_LOOPS_PASSES: passes always; an explicit
  * depth or tile (wf_set_blocking, wf_set_tiles) selects it too.  Results do
  * not depend on the mode, but for what is not finite: a pass of several pressure
  * sweeps carries the NaN of a fluid cell without fluid neighbours through walls of up to

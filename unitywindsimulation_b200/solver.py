@@ -283,8 +283,8 @@ class FvmSolverCuda:
         self._check(self._lib.wf_set_blocking(self._h, int(pres_k), int(vel_k)))
 
     def set_loops(self, mode: int) -> None:
-        """_lib.LOOPS_AUTO (loops whose grid fits on chip run as one launch,
-        the default) or _lib.LOOPS_PASSES (wf_set_loops)."""
+        """_lib.LOOPS_AUTO (loops whose grid fits on chip run as one launch
+        where that is faster, the default) or _lib.LOOPS_PASSES (wf_set_loops)."""
         self._check(self._lib.wf_set_loops(self._h, int(mode)))
 
     def loop_plan(self, kernel: int, beside: bool = False):
